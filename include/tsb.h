@@ -90,6 +90,16 @@ int tsb_nl_build(const void *positions, const void *cell_row, const uint8_t *pbc
                  int64_t mapping_stride, int64_t *system_mapping, void *shifts,
                  int64_t capacity, int64_t *n_pairs, void *workspace,
                  size_t workspace_bytes, void *stream);
+/* The same list with the two mapping rows back to back: mapping (room for
+ * 2 * capacity) holds row 0 at [0, P) and row 1 at [P, 2 P), P = *n_pairs, so the
+ * caller views it as [2, P] without a copy.  When P exceeds `capacity` nothing is
+ * written. */
+int tsb_nl_build_packed(const void *positions, const void *cell_row, const uint8_t *pbc,
+                        const int64_t *system_idx, int64_t n_atoms, int64_t n_systems,
+                        int dtype, double cutoff, int flags, int64_t *mapping,
+                        int64_t *system_mapping, void *shifts, int64_t capacity,
+                        int64_t *n_pairs, void *workspace, size_t workspace_bytes,
+                        void *stream);
 
 /* ---- pair potential energy / forces / virial -----------------------------
  * Replaces PairPotentialModel.forward (torch_sim/models/pair_potential.py:351-464)

@@ -12,7 +12,7 @@
 // c_k -> (bin c_k mod nb_k, image floor(c_k / nb_k)) on periodic axes.  That
 // covers all images the reference replicates (get_cell_shift_idx,
 // transforms.py:470-497) for any cell, including cells smaller than rc.
-#include "tsb_common.cuh"
+#include "tsb_window.cuh"
 
 namespace tsb {
 
@@ -322,7 +322,8 @@ __global__ void k_bin_scatter(const int32_t *bin_of, const int64_t *bin_start,
 // Deterministic order inside each bin (ascending atom index), then gather the
 // wrapped positions into bin order.
 __global__ void k_bin_sort(const int64_t *bin_start, int64_t nbins_total, int32_t *sidx,
-                           const double4 *wpos, const int32_t *species, double4 *spos) {
+                           const double4 *wpos, const int32_t *species, double4 *spos,
+                           int32_t *sbin) {
   int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nbins_total) return;
   int64_t s0 = bin_start[b], s1 = bin_start[b + 1];
@@ -341,6 +342,7 @@ __global__ void k_bin_sort(const int64_t *bin_start, int64_t nbins_total, int32_
     const unsigned long long hi = species ? (unsigned long long)(uint32_t)species[j] : 0ull;
     w.w = __longlong_as_double((long long)((hi << 32) | (uint32_t)j));
     spos[p] = w;
+    sbin[p] = (int32_t)b;
   }
 }
 
@@ -442,6 +444,7 @@ __global__ void __launch_bounds__(kBlock)
       const int64_t slot = start + at + rank;
       b.spos[slot] = wv4;
       b.sidx[slot] = (int32_t)i;
+      b.sbin[slot] = (int32_t)base + lb;
     }
   }
 }
@@ -495,6 +498,7 @@ void carve_bins(Carver &c, BinData &b, int64_t n, int64_t ns) {
   b.spos = c.take<double4>(n);
   b.wpos = c.take<double4>(n);
   b.sidx = c.take<int32_t>(n);
+  b.sbin = c.take<int32_t>(n);
   b.bin_count = c.take<int32_t>(b.bcap);
   b.bin_start = c.take<int64_t>(b.bcap + 1);
   b.bin_fill = c.take<int32_t>(b.bcap);
@@ -528,7 +532,7 @@ int prepare_bins(const P *positions, const P *cell_row, const uint8_t *pbc,
     k_bin_scatter<<<grid_for(n), kBlock, 0, st>>>(b.bin_of, b.bin_start, b.bin_fill, n,
                                                   b.sidx);
     k_bin_sort<<<grid_for(b.bcap), kBlock, 0, st>>>(b.bin_start, b.bcap, b.sidx, b.wpos,
-                                                    species, b.spos);
+                                                    species, b.spos, b.sbin);
   }
   TSB_CHECK_LAUNCH();
   return TSB_OK;
@@ -540,5 +544,131 @@ template int prepare_bins<float>(const float *, const float *, const uint8_t *,
 template int prepare_bins<double>(const double *, const double *, const uint8_t *,
                                   const int64_t *, int64_t, int64_t, double, BinData &,
                                   cudaStream_t, const int32_t *);
+
+// Systems of at most this many columns put their columns one after another, so that
+// tiles run across them and only a system's last one is short; a larger system
+// starts a tile at every column.
+constexpr int kTileColumns = 64;
+
+// Column order and tiles.  A warp looks at 32 slots; the first slot of a column (the
+// first atom of its first non-empty row) makes the warp lay the column out: lane z
+// takes the bins at z of the column's rows.  Odd columns run backwards, so that the
+// order turns round at their ends.
+__global__ void k_window_tiles(BinData b, int64_t n, const uint8_t *sys_active, TileList t) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // is this lane's slot the first of its column?
+  bool lead = false;
+  int s = 0, x0 = 0, y0 = 0, gx = 1, gy = 1;
+  if (p < n) {
+    const int bin = b.sbin[p];
+    s = b.sys_of[b.sidx[p]];
+    const SysGeom &G = b.geom[s];
+    const int lb = bin - G.bin_base, row = lb / G.nb[2], x = row / G.nb[1], y = row % G.nb[1];
+    const int row0 = bin - lb % G.nb[2];
+    if (b.bin_start[row0] == p && (!sys_active || sys_active[s])) {
+      column_dims(G, gx, gy);
+      x0 = x / gx * gx;
+      y0 = y / gy * gy;
+      lead = true;
+      for (int xx = x0; xx <= x; ++xx)
+        for (int yy = y0; yy < min(y0 + gy, G.nb[1]); ++yy)
+          if (xx < x || yy < y) {
+            const int r = G.bin_base + (xx * G.nb[1] + yy) * G.nb[2];
+            lead = lead && b.bin_start[r] == b.bin_start[r + G.nb[2]];
+          }
+    }
+  }
+  for (unsigned m = __ballot_sync(full, lead); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    const int cs = __shfl_sync(full, s, src);
+    const int cx = __shfl_sync(full, x0, src), cy = __shfl_sync(full, y0, src);
+    const int dx = __shfl_sync(full, gx, src), dy = __shfl_sync(full, gy, src);
+    const SysGeom &G = b.geom[cs];
+    const int nb0 = G.nb[0], nb1 = G.nb[1], nb2 = G.nb[2];
+    const int nx = min(dx, nb0 - cx), ny = min(dy, nb1 - cy);
+    auto row_of = [&](int r) {  // first bin of the column's row r < nx ny
+      return G.bin_base + ((cx + r / ny) * nb1 + cy + r % ny) * nb2;
+    };
+    int total = 0;
+    for (int r = 0; r < nx * ny; ++r)
+      total += (int)(b.bin_start[row_of(r) + nb2] - b.bin_start[row_of(r)]);
+    const int ncy = (nb1 + dy - 1) / dy, ncx = (nb0 + dx - 1) / dx;
+    const int col = cx / dx * ncy + cy / dy;
+    const bool joined = ncx * ncy <= kTileColumns;
+    // where the column goes in the system's part of the order
+    int at = 0;
+    if (joined) {
+      for (int c = lane; c < col; c += 32)  // atoms in the columns before
+        for (int xx = c / ncy * dx; xx < min(c / ncy * dx + dx, nb0); ++xx) {
+          const int ya = c % ncy * dy, yb = min(ya + dy, nb1);
+          const int r = G.bin_base + (xx * nb1 + ya) * nb2;
+          at += (int)(b.bin_start[r + (yb - ya) * nb2] - b.bin_start[r]);
+        }
+      at = __reduce_add_sync(full, at);
+    } else {
+      if (lane == 0) at = atomicAdd(&t.cursor[cs], total);
+      at = __shfl_sync(full, at, 0);
+    }
+    const int base = (int)G.start;
+    const bool back = joined && (col & 1);
+    int done = at;
+    for (int z0 = 0; z0 < nb2; z0 += 32) {
+      const int zz = z0 + lane, z = back ? nb2 - 1 - zz : zz;
+      int c = 0;
+      if (zz < nb2)
+        for (int r = 0; r < nx * ny; ++r)
+          c += (int)(b.bin_start[row_of(r) + z + 1] - b.bin_start[row_of(r) + z]);
+      int inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(full, inc, o);
+        if (lane >= o) inc += u;
+      }
+      if (zz < nb2) {
+        int32_t *out = t.order + base + done + inc - c;
+        for (int r = 0; r < nx * ny; ++r) {
+          const int q1 = (int)b.bin_start[row_of(r) + z + 1];
+          for (int q = (int)b.bin_start[row_of(r) + z]; q < q1; ++q) *out++ = q;
+        }
+      }
+      done += __shfl_sync(full, inc, 31);
+    }
+    // tiles that start in the column
+    const int first = joined ? (at + 31) / 32 * 32 : at;
+    const int end = at + total, limit = joined ? G.count : end;
+    const int nt = first < end ? (end - first + 31) / 32 : 0;
+    int k0 = 0;
+    if (lane == 0 && nt > 0) k0 = atomicAdd(t.n_tiles, nt);
+    k0 = __shfl_sync(full, k0, 0);
+    for (int k = lane; k < nt; k += 32) {
+      const int o = first + 32 * k;
+      t.tiles[k0 + k] = Tile{base + o, min(32, limit - o), cs};
+    }
+  }
+}
+
+void carve_tiles(Carver &c, TileList &t, int64_t n, int64_t ns) {
+  t.tiles = c.take<Tile>(n);
+  t.n_tiles = c.take<int32_t>(2);
+  t.order = c.take<int32_t>(n);
+  t.cursor = c.take<int32_t>(ns);
+}
+
+int restart_tiles(const TileList &t, cudaStream_t st) {
+  cudaMemsetAsync(t.n_tiles + 1, 0, sizeof(int32_t), st);
+  TSB_CHECK_LAUNCH();
+  return TSB_OK;
+}
+
+int window_tiles(const BinData &b, int64_t n, int64_t ns, const uint8_t *sys_active,
+                 const TileList &t, cudaStream_t st) {
+  cudaMemsetAsync(t.n_tiles, 0, 2 * sizeof(int32_t), st);
+  cudaMemsetAsync(t.cursor, 0, sizeof(int32_t) * ns, st);
+  k_window_tiles<<<grid_for(n), kBlock, 0, st>>>(b, n, sys_active, t);
+  TSB_CHECK_LAUNCH();
+  return TSB_OK;
+}
 
 }  // namespace tsb

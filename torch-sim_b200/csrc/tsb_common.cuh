@@ -103,6 +103,7 @@ struct BinData {
   double4 *spos;        // [N] wrapped position in bin order; .w = atom index bits
   double4 *wpos;        // [N] wrapped position in atom order (scratch)
   int32_t *sidx;        // [N] atom index in bin order
+  int32_t *sbin;        // [N] bin of each slot of the bin order
   int32_t *bin_count;   // [Bcap]
   int64_t *bin_start;   // [Bcap+1]
   int32_t *bin_fill;    // [Bcap]
@@ -147,5 +148,20 @@ int prepare_bins_any(const P *positions, const P *cell_row, const uint8_t *pbc,
                      const int64_t *system_idx, int64_t n_atoms, int64_t n_systems,
                      double search_cutoff, BinData &b, cudaStream_t st, const int32_t *species,
                      int64_t max_system_atoms);
+
+// Tiles of up to 32 neighbouring atoms for the tile-per-warp kernels
+// (tsb_window.cuh): tiles[0..*n_tiles) of the active systems, in any order (a tile's
+// results do not depend on it).
+struct Tile;
+struct TileList {
+  Tile *tiles;       // [N]
+  int32_t *n_tiles;  // [2]: tiles, and the next one to work on
+  int32_t *order;    // [N] slots in column order
+  int32_t *cursor;   // [S]
+};
+void carve_tiles(Carver &c, TileList &t, int64_t n_atoms, int64_t n_systems);
+int restart_tiles(const TileList &t, cudaStream_t st);  // before another pass over them
+int window_tiles(const BinData &b, int64_t n_atoms, int64_t n_systems, const uint8_t *sys_active,
+                 const TileList &t, cudaStream_t st);
 
 }  // namespace tsb

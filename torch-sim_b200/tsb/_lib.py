@@ -44,6 +44,8 @@ PROTOTYPES = {
     "tsb_nl_workspace_size": (_sz, [_i64, _i64]),
     "tsb_nl_build": (_int, [_vp, _vp, _vp, _vp, _i64, _i64, _int, _dbl, _int, _vp, _i64,
                             _vp, _vp, _i64, _vp, _vp, _sz, _vp]),
+    "tsb_nl_build_packed": (_int, [_vp, _vp, _vp, _vp, _i64, _i64, _int, _dbl, _int, _vp,
+                                   _vp, _vp, _i64, _vp, _vp, _sz, _vp]),
     "tsb_pair_workspace_size": (_sz, [_i64, _i64]),
     "tsb_pair_forward": (_int, [_int, _vp, _int, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _int,
                                 _dbl, _int, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _sz,

@@ -64,18 +64,18 @@ def _nl_build(positions, cell_row, pbc, system_idx, cutoff, flags, n_systems, ca
     n_pairs = torch.zeros(1, dtype=torch.int64, device=dev)
     cap = int(capacity)
     for _ in range(2):
-        mapping = torch.empty((2, max(cap, 1)), dtype=torch.int64, device=dev)
+        mapping = torch.empty(2 * max(cap, 1), dtype=torch.int64, device=dev)
         sysmap = torch.empty(max(cap, 1), dtype=torch.int64, device=dev)
         shifts = torch.empty((max(cap, 1), 3), dtype=dt, device=dev)
-        L.call("tsb_nl_build", _P(positions), _P(cell_row), _P(pbc), _P(system_idx), n,
-               n_systems, L.dtype_code(dt), float(cutoff), int(flags), _P(mapping),
-               mapping.shape[1], _P(sysmap), _P(shifts), cap, _P(n_pairs), _P(ws), ws.numel(),
-               _stream(positions))
+        L.call("tsb_nl_build_packed", _P(positions), _P(cell_row), _P(pbc), _P(system_idx), n,
+               n_systems, L.dtype_code(dt), float(cutoff), int(flags), _P(mapping), _P(sysmap),
+               _P(shifts), cap, _P(n_pairs), _P(ws), ws.numel(), _stream(positions))
         p = int(n_pairs.item())
         if p <= cap:
             break
         cap = int(p * 1.15) + 16
-    return mapping[:, :p].contiguous(), sysmap[:p].contiguous(), shifts[:p].contiguous()
+    # the rows lie back to back at the pair count: views, no copies
+    return mapping[:2 * p].view(2, p), sysmap[:p], shifts[:p]
 
 
 def _nl_build_fake(positions, cell_row, pbc, system_idx, cutoff, flags, n_systems, capacity):
