@@ -1,120 +1,266 @@
 // Fused neighbour search + pair energy/force/virial (drop-in for
 // PairPotentialModel.forward, torch_sim/models/pair_potential.py:351-464).
 //
-// One thread per atom i (launched in bin order so neighbouring threads share
-// candidate bins in L1/L2) walks the full neighbour set of i, so forces need no
-// atomics and the summation order is fixed (deterministic results).  Each
-// unordered pair is evaluated from both ends; per-atom energies/virials take
+// A warp works through the full neighbour set of an atom (candidates gathered by
+// tsb_window.cuh), so forces need no atomics and the summation order is fixed
+// (deterministic results).  Each unordered pair is evaluated from both ends; per-atom energies/virials take
 // half of each visit, matching the half-list weights of pair_potential.py:402-441.
 // Displacements are formed in FP64 from the wrapped FP64 positions; the pair
 // function runs in R (float by default, double with TSB_MATH_FP64).
 #include "tsb_pair.cuh"
-#include "tsb_search.cuh"
 #include "tsb_sysreduce.cuh"
+#include "tsb_window.cuh"
 
 namespace tsb {
 
-// LANES > 1: LANES lanes per atom (small batches; lanes split the candidates and the
-// partial sums are reduced in a fixed order), LANES = 1: one thread per atom.
-template <int POT, class R, class P, int LANES>
-__global__ void __launch_bounds__(128)
-    k_pair_forces(BinData b, int64_t n, const double *__restrict__ table, int ns_species,
-                  const int32_t *__restrict__ species, double cutoff, int flags, P *forces,
-                  P *energies, P *stresses, double *e_half, double *vir_half,
-                  const uint8_t *__restrict__ sys_active) {
-  __shared__ PairPrm<R> prm[kMaxSpecies * kMaxSpecies];
-  __shared__ double prc2[kMaxSpecies * kMaxSpecies];
-  for (int k = threadIdx.x; k < ns_species * ns_species; k += blockDim.x) {
+// One pair's terms, added to a lane's sums: forces in R, energy and virial in FP64
+// (R is FP32 by default; the per-system sums are FP64).
+//
+// ROUND: the FP32 force sums round each product and sum on its own (FP32 pair math
+// with FP64 results, whose digits show it); else they may use one fused step.
+template <int POT, class R, bool VIR, bool ROUND>
+struct PairSum {
+  R fx, fy, fz;
+  double ei, v[VIR ? 6 : 1];
+
+  __device__ __forceinline__ void clear() {
+    fx = fy = fz = 0;
+    ei = 0.0;
+#pragma unroll
+    for (int k = 0; k < (VIR ? 6 : 1); ++k) v[k] = 0.0;
+  }
+
+  // adds the pair when `on` (a pair left out is evaluated all the same and its terms
+  // replaced by zeros, so that the lanes of a warp stay together); returns fr
+  template <bool FORCE = true>
+  __device__ __forceinline__ R add(bool on, R rx, R ry, R rz, const PairPrm<R> &ij,
+                                   const PairPrm<R> &ji) {
+    const R r2 = rx * rx + ry * ry + rz * rz;
+    R e, fr;  // fr = -(dV/dr)/r
+    pair_eval<POT, R>(ij, r2, e, fr);
+    // force-defined pairs: both directed pairs (i, j) and (j, i) of the reference's
+    // full list act on i, so the force adds f_ij and f_ji and the virial takes half
+    // of it (pair_potential.py:567-600, stress scale 1/2 for a full list)
+    double vw = 1.0;
+    if constexpr (POT == TSB_POT_PLIFE) {
+      R e2, fr2;
+      pair_eval<POT, R>(ji, r2, e2, fr2);
+      fr += fr2;
+      vw = 0.5;
+    }
+    fr = on ? fr : R(0);
+    e = on ? e : R(0);
+    const R gx = fr * rx, gy = fr * ry, gz = fr * rz;  // force on j
+    if constexpr (FORCE && ROUND) {
+      fx = __fsub_rn(fx, __fmul_rn(fr, rx));
+      fy = __fsub_rn(fy, __fmul_rn(fr, ry));
+      fz = __fsub_rn(fz, __fmul_rn(fr, rz));
+    } else if constexpr (FORCE) {
+      fx -= gx;
+      fy -= gy;
+      fz -= gz;
+    }
+    ei += (double)e;
+    if constexpr (VIR) {
+      v[0] += vw * (double)(rx * gx);
+      v[1] += vw * (double)(ry * gy);
+      v[2] += vw * (double)(rz * gz);
+      v[3] += vw * (double)(ry * gz);
+      v[4] += vw * (double)(rx * gz);
+      v[5] += vw * (double)(rx * gy);
+    }
+    return fr;
+  }
+};
+
+// results of atom i from its sums t[0..NA)
+template <class P, bool VIR>
+__device__ __forceinline__ void write_atom(int64_t i, const double *t, int flags, double vol,
+                                           P *forces, P *energies, P *stresses, double *e_half,
+                                           double *vir_half) {
+  if (flags & TSB_OUT_FORCES)
+    for (int c = 0; c < 3; ++c) forces[3 * i + c] = (P)t[c];
+  // reference per-atom energies: each endpoint receives the full pair energy
+  // (pair_potential.py:411-417 with weight 1 on both mapping rows)
+  if (flags & TSB_OUT_ENERGIES) energies[i] = (P)t[3];
+  e_half[i] = 0.5 * t[3];
+  if constexpr (VIR) {
+    for (int c = 0; c < 6; ++c) vir_half[6 * i + c] = 0.5 * t[4 + c];
+    if (flags & TSB_OUT_STRESSES) {
+      // per-atom stress: -1/2 sum_j r_ij (x) f_ij / V (pair_potential.py:262-272)
+      const double c = -0.5 / vol;
+      P *o = stresses + 9 * i;
+      o[0] = (P)(c * t[4]); o[1] = (P)(c * t[9]); o[2] = (P)(c * t[8]);
+      o[3] = (P)(c * t[9]); o[4] = (P)(c * t[5]); o[5] = (P)(c * t[7]);
+      o[6] = (P)(c * t[8]); o[7] = (P)(c * t[7]); o[8] = (P)(c * t[6]);
+    }
+  }
+}
+
+template <class R, class P, bool VIR>
+struct PairWarpSmem {
+  // FP32 pair math with FP64 results: the FP32 force sums decide the result's
+  // digits, so their order is kept: four partial sums per component, each over every
+  // fourth candidate of a span in turn, as four lanes per atom would take them
+  static constexpr bool ORDERED = sizeof(R) == 4 && sizeof(P) == 8;
+  static constexpr int NA = VIR ? 10 : 4;  // forces, energy, virial
+  WinSmem win;
+  float4 term[ORDERED ? 32 : 1];
+  double acc[NA];
+  uint8_t tag[32];
+};
+
+// Small calls: one warp per atom, every atom of the batch in flight at once.  Lanes
+// are added in FP64 by exchange.  (LJ, 256 atoms, FP64: 10.1 us against 57.4 us with
+// four lanes walking an atom's rows in turn.)
+template <int POT, class R, class P, bool VIR>
+__global__ void __launch_bounds__(32 * kWinWarps)
+    k_pair_warp(BinData b, int64_t n, const double *__restrict__ table, int nsp, double cutoff,
+                int flags, P *forces, P *energies, P *stresses, double *e_half,
+                double *vir_half, const uint8_t *__restrict__ sys_active) {
+  using Warp = PairWarpSmem<R, P, VIR>;
+  constexpr bool ORDERED = Warp::ORDERED;
+  constexpr int NV = VIR ? 16 : 4;
+  extern __shared__ __align__(16) char smem[];
+  Warp *warps = (Warp *)smem;
+  PairPrm<R> *prm = (PairPrm<R> *)(warps + kWinWarps);
+  double *prc2 = (double *)(prm + nsp * nsp);
+  for (int k = threadIdx.x; k < nsp * nsp; k += blockDim.x) {
     prm[k] = make_prm<R>(POT, table + 5 * k, cutoff);
     prc2[k] = pair_rc2(POT, table + 5 * k, cutoff);
   }
   __syncthreads();
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t p = t / LANES;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  Warp &me = warps[threadIdx.x >> 5];
+  const int64_t p = (int64_t)blockIdx.x * kWinWarps + (threadIdx.x >> 5);
   if (p >= n) return;
   const double4 w = b.spos[p];
   const int i = tag_atom(w.w);
   const int s = b.sys_of[i];
   if (sys_active && !sys_active[s]) return;
   const SysGeom &G = b.geom[s];
-  const int si = min(max(tag_species(w.w), 0), ns_species - 1);
-  const PairPrm<R> *row = prm + si * ns_species;
-  // forces accumulate in R; energy and virial in FP64 (per-system sums in FP64)
-  R fx = 0, fy = 0, fz = 0;
-  double ei = 0, vxx = 0, vyy = 0, vzz = 0, vyz = 0, vxz = 0, vxy = 0;
-  auto pair = [&](int, int, int, int, double dx, double dy, double dz, double d2,
-                       int sp) {
-                     const int sj = min(max(sp, 0), ns_species - 1);
-                     if (!(d2 < prc2[si * ns_species + sj])) return;  // FP64 decision
-                     const PairPrm<R> &q = row[sj];
-                     const R rx = (R)dx, ry = (R)dy, rz = (R)dz;
-                     const R r2 = rx * rx + ry * ry + rz * rz;
-                     R e, fr;
-                     pair_eval<POT, R>(q, r2, e, fr);
-                     // force-defined pairs: i's thread sees both directed pairs
-                     // (i, j) and (j, i) of the reference's full list, so the force
-                     // adds f_ij and f_ji and the virial takes half of it
-                     // (pair_potential.py:567-600, stress scale 1/2 for a full list)
-                     double vw = 1.0;
-                     if constexpr (POT == TSB_POT_PLIFE) {
-                       R e2, fr2;
-                       pair_eval<POT, R>(prm[sj * ns_species + si], r2, e2, fr2);
-                       fr += fr2;
-                       vw = 0.5;
-                     }
-                     const R gx = fr * rx, gy = fr * ry, gz = fr * rz;  // force on j
-                     fx -= gx;
-                     fy -= gy;
-                     fz -= gz;
-                     ei += (double)e;
-                     vxx += vw * (double)(rx * gx);
-                     vyy += vw * (double)(ry * gy);
-                     vzz += vw * (double)(rz * gz);
-                     vyz += vw * (double)(ry * gz);
-                     vxz += vw * (double)(rx * gz);
-                     vxy += vw * (double)(rx * gy);
-                   };
-  if constexpr (LANES > 1) {
-    group_search_neighbors<LANES>(G, b.spos, b.bin_start, i, w.x, w.y, w.z, cutoff * cutoff, false,
-                          pair);
-    fx = group_sum<LANES>(fx);
-    fy = group_sum<LANES>(fy);
-    fz = group_sum<LANES>(fz);
-    ei = group_sum<LANES>(ei);
-    vxx = group_sum<LANES>(vxx);
-    vyy = group_sum<LANES>(vyy);
-    vzz = group_sum<LANES>(vzz);
-    vyz = group_sum<LANES>(vyz);
-    vxz = group_sum<LANES>(vxz);
-    vxy = group_sum<LANES>(vxy);
-    if ((threadIdx.x & (LANES - 1)) != 0) return;
-  } else {
-    search_neighbors(G, b.spos, b.bin_start, i, w.x, w.y, w.z, cutoff * cutoff, false, pair);
+  const int si = min(max(tag_species(w.w), 0), nsp - 1);
+  PairSum<POT, R, VIR, false> sum;
+  sum.clear();
+  float fo = 0.0f;  // ORDERED, lanes 0..11: component lane / 4, partial sum lane % 4
+  WinSmem &S = me.win;
+  window_gather(S, G, b.spos, b.bin_start, w, cutoff, [&](int kept) {
+    for (int t0 = 0; t0 < kept; t0 += 32) {
+      const int t = t0 + lane;
+      float4 term = make_float4(0.f, 0.f, 0.f, 0.f);
+      int share = 0;
+      if (t < kept) {
+        const double dx = S.x[t] - w.x, dy = S.y[t] - w.y, dz = S.z[t] - w.z;
+        const int info = S.info[t], sj = min(info & 255, nsp - 1);
+        share = (info >> 9) & 3;
+        if (dx * dx + dy * dy + dz * dz < prc2[si * nsp + sj] &&  // FP64 decision
+            !(S.q[t] == p && (info & 256))) {
+          const R fr = sum.template add<!ORDERED>(true, (R)dx, (R)dy, (R)dz,
+                                                  prm[si * nsp + sj], prm[sj * nsp + si]);
+          if constexpr (ORDERED) term = make_float4((float)dx, (float)dy, (float)dz, fr);
+        }
+      }
+      if constexpr (ORDERED) {
+        __syncwarp();
+        me.term[lane] = term;
+        me.tag[lane] = (uint8_t)share;
+        __syncwarp();
+        if (lane < 12) {
+          const int c = min(kept - t0, 32);
+          const float *d = &me.term[0].x + lane / 4;
+          for (int k = 0; k < c; ++k)
+            if (me.tag[k] == (lane & 3)) fo = __fsub_rn(fo, __fmul_rn(me.term[k].w, d[4 * k]));
+        }
+      }
+    }
+  });
+  double v[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
+  v[0] = (double)sum.fx;
+  v[1] = (double)sum.fy;
+  v[2] = (double)sum.fz;
+  v[3] = sum.ei;
+  if constexpr (VIR)
+    for (int k = 0; k < 6; ++k) v[4 + k] = sum.v[k];
+  const double tot = warp_multi_sum<NV>(v);
+  constexpr int W = 32 / NV;
+  if (lane % W == 0 && lane / W < Warp::NA) me.acc[lane / W] = tot;
+  if constexpr (ORDERED) {
+    const int l = 4 * (lane % 3);
+    const float a0 = __shfl_sync(full, fo, l), a1 = __shfl_sync(full, fo, l + 1);
+    const float a2 = __shfl_sync(full, fo, l + 2), a3 = __shfl_sync(full, fo, l + 3);
+    __syncwarp();
+    if (lane < 3) me.acc[lane] = (double)((a0 + a2) + (a1 + a3));
   }
-  if (flags & TSB_OUT_FORCES) {
-    forces[3 * i] = (P)fx;
-    forces[3 * i + 1] = (P)fy;
-    forces[3 * i + 2] = (P)fz;
+  __syncwarp();
+  if (lane == 0)
+    write_atom<P, VIR>(i, me.acc, flags, G.vol, forces, energies, stresses, e_half, vir_half);
+}
+
+// Large calls: one warp per tile, one lane per atom.  MONO: one species, whose row of
+// the table stays in registers.
+template <int POT, class R, class P, bool VIR, bool MONO>
+__global__ void __launch_bounds__(32 * kWinWarps, sizeof(R) == 4 ? 6 : 4)
+    k_pair_tile(BinData b, TileList tl, const double *__restrict__ table, int nsp, double cutoff, int flags, P *forces,
+                P *energies, P *stresses, double *e_half, double *vir_half) {
+  constexpr bool ROUND = sizeof(R) == 4 && sizeof(P) == 8;  // sums in search order
+  extern __shared__ __align__(16) char smem[];
+  TileSmem<false> *warps = (TileSmem<false> *)smem;
+  PairPrm<R> *prm = (PairPrm<R> *)(warps + kWinWarps);
+  double *prc2 = (double *)(prm + nsp * nsp);
+  for (int k = threadIdx.x; k < nsp * nsp; k += blockDim.x) {
+    prm[k] = make_prm<R>(POT, table + 5 * k, cutoff);
+    prc2[k] = pair_rc2(POT, table + 5 * k, cutoff);
   }
-  // reference per-atom energies: each endpoint receives the full pair energy
-  // (pair_potential.py:411-417 with weight 1 on both mapping rows)
-  if (flags & TSB_OUT_ENERGIES) energies[i] = (P)ei;
-  if (flags & TSB_OUT_STRESSES) {
-    // per-atom stress: -1/2 sum_j r_ij (x) f_ij / V (pair_potential.py:262-272)
-    const double c = -0.5 / G.vol;
-    P *o = stresses + 9 * i;
-    o[0] = (P)(c * vxx); o[1] = (P)(c * vxy); o[2] = (P)(c * vxz);
-    o[3] = (P)(c * vxy); o[4] = (P)(c * vyy); o[5] = (P)(c * vyz);
-    o[6] = (P)(c * vxz); o[7] = (P)(c * vyz); o[8] = (P)(c * vzz);
+  __syncthreads();
+  const int wid = threadIdx.x >> 5;
+  TileSmem<false> &S = warps[wid];
+  const PairPrm<R> row0 = prm[0];
+  const double rc2_0 = prc2[0];
+  const int nt = *tl.n_tiles;
+  TileQueue queue(tl);
+  for (int g; (g = queue.take(tl, nt)) >= 0;) {
+    const Tile T = tl.tiles[g];
+    PairSum<POT, R, VIR, ROUND> sum;
+    int si = 0;
+    tile_gather<!ROUND>(
+        S, b, T, tl.order, nullptr, cutoff,
+        [&](const TileAtom &A) {
+          sum.clear();
+          si = min(max(tag_species(A.w.w), 0), nsp - 1);
+        },
+        [&](const TileAtom &A, int kept, float pre2) {
+          for (int t0 = 0; t0 < kept;) {
+            int nn, unused = 0;
+            t0 = tile_scan<false>(S, A, t0, kept, pre2, nn, 0.0f, unused);
+            const int most = __reduce_max_sync(0xffffffffu, nn);
+            const uint8_t *note = S.note + (threadIdx.x & 31);
+#pragma unroll sizeof(R) == 4 ? 2 : 1
+            for (int k = 0; k < most; ++k) {
+              bool on = k < nn;
+              const int t = on ? note[k * kTileStride] : 0;
+              const double dx = S.x[t] - A.w.x, dy = S.y[t] - A.w.y, dz = S.z[t] - A.w.z;
+              const double d2 = dx * dx + dy * dy + dz * dz;
+              const int sj = MONO ? 0 : min((int)S.spec[t], nsp - 1);
+              on = on && d2 < (MONO ? rc2_0 : prc2[si * nsp + sj]) &&  // FP64 decision
+                   !(d2 == 0.0 && S.j[t] == A.i);
+              sum.add(on, (R)dx, (R)dy, (R)dz, MONO ? row0 : prm[si * nsp + sj],
+                      MONO ? row0 : prm[sj * nsp + si]);
+            }
+            __syncwarp();
+          }
+        },
+        [&](const TileAtom &A) {
+          if (!A.have) return;
+          double t[VIR ? 10 : 4] = {(double)sum.fx, (double)sum.fy, (double)sum.fz, sum.ei};
+          if constexpr (VIR)
+            for (int k = 0; k < 6; ++k) t[4 + k] = sum.v[k];
+          write_atom<P, VIR>(tag_atom(A.w.w), t, flags, b.geom[T.sys].vol, forces, energies, stresses,
+                             e_half, vir_half);
+        });
   }
-  e_half[i] = 0.5 * ei;
-  double *v = vir_half + 6 * i;
-  v[0] = 0.5 * vxx;
-  v[1] = 0.5 * vyy;
-  v[2] = 0.5 * vzz;
-  v[3] = 0.5 * vyz;
-  v[4] = 0.5 * vxz;
-  v[5] = 0.5 * vxy;
 }
 
 struct PairWork {
@@ -123,6 +269,7 @@ struct PairWork {
   double *vir_half;
   double *part;  // [7 * ns * chunks] slice sums (chunks > 1 only)
   int chunks;
+  TileList tl;  // large calls
 };
 
 static void carve_pair(Carver &c, PairWork &w, int64_t n, int64_t ns) {
@@ -131,20 +278,45 @@ static void carve_pair(Carver &c, PairWork &w, int64_t n, int64_t ns) {
   w.vir_half = c.take<double>(6 * n);
   w.chunks = reduce_chunks(n, ns);
   w.part = w.chunks > 1 ? c.take<double>(7 * ns * w.chunks) : nullptr;
+  carve_tiles(c, w.tl, n, ns);
 }
 
-template <int POT, class R, class P>
-static void launch_forces(PairWork &w, int64_t n, const double *table, int nsp,
-                          const int32_t *species, double cutoff, int flags, P *forces,
-                          P *energies, P *stresses, const uint8_t *active, cudaStream_t st) {
-  if (n <= kGroupSearchMaxAtoms)
-    k_pair_forces<POT, R, P, kSearchGroup><<<grid_for(kSearchGroup * n, 128), 128, 0, st>>>(
-        w.b, n, table, nsp, species, cutoff, flags, forces, energies, stresses, w.e_half,
-        w.vir_half, active);
-  else
-    k_pair_forces<POT, R, P, 1><<<grid_for(n, 128), 128, 0, st>>>(
-        w.b, n, table, nsp, species, cutoff, flags, forces, energies, stresses, w.e_half,
-        w.vir_half, active);
+// Up to this many atoms a call takes one warp per atom: fewer tiles than that leave
+// most of the GPU's resident warps idle.  With FP32 pair math and FP64 results the
+// limit is that of the four-lane order of the FP32 sums (k_pair_warp keeps the
+// four-lane order, k_pair_tile the one-lane order that larger calls have).
+constexpr int64_t kPairWarpMaxAtoms = 16384;
+
+template <int POT, class R, class P, bool VIR>
+static void launch_forces(PairWork &w, int64_t n, int64_t ns, const double *table, int nsp, double cutoff,
+                          int flags, P *forces, P *energies, P *stresses,
+                          const uint8_t *active, cudaStream_t st) {
+  using Warp = PairWarpSmem<R, P, VIR>;
+  const size_t tab = (size_t)nsp * nsp * (sizeof(PairPrm<R>) + sizeof(double));
+  auto room = [](auto kernel, size_t bytes) {
+    if (bytes > 48 * 1024)
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return bytes;
+  };
+  if (n <= (Warp::ORDERED ? kGroupSearchMaxAtoms : kPairWarpMaxAtoms)) {
+    auto kernel = k_pair_warp<POT, R, P, VIR>;
+    kernel<<<grid_for(n, kWinWarps), 32 * kWinWarps, 
+             room(kernel, kWinWarps * sizeof(Warp) + tab), st>>>(
+        w.b, n, table, nsp, cutoff, flags, forces, energies, stresses, w.e_half, w.vir_half,
+        active);
+  } else {
+    window_tiles(w.b, n, ns, active, w.tl, st);
+    auto go = [&](auto kernel) {
+      const size_t bytes = room(kernel, kWinWarps * sizeof(TileSmem<false>) + tab);
+      kernel<<<tile_grid(kernel, bytes), 32 * kWinWarps, bytes, st>>>(
+          w.b, w.tl, table, nsp, cutoff, flags, forces, energies, stresses, w.e_half,
+          w.vir_half);
+    };
+    if (nsp == 1)
+      go(k_pair_tile<POT, R, P, VIR, true>);
+    else
+      go(k_pair_tile<POT, R, P, VIR, false>);
+  }
 }
 
 template <class P>
@@ -157,23 +329,29 @@ static int pair_forward(int pot, const double *table, int nsp, const int32_t *sp
   TSB_TRY(prepare_bins_any<P>(pos, cell, pbc, sys, n, ns, cutoff, w.b, st, species, max_sys));
   const bool f64 = flags & TSB_MATH_FP64;
   if (n > 0) {
-#define TSB_LAUNCH(POT)                                                                    \
-  if (f64)                                                                                 \
-    launch_forces<POT, double, P>(w, n, table, nsp, species, cutoff, flags, forces,       \
-                                  energies, stresses, active, st);                         \
-  else                                                                                     \
-    launch_forces<POT, float, P>(w, n, table, nsp, species, cutoff, flags, forces,        \
-                                 energies, stresses, active, st);
-    if (pot == TSB_POT_LJ) {
-      TSB_LAUNCH(TSB_POT_LJ)
-    } else if (pot == TSB_POT_MORSE) {
-      TSB_LAUNCH(TSB_POT_MORSE)
-    } else if (pot == TSB_POT_SOFT) {
-      TSB_LAUNCH(TSB_POT_SOFT)
-    } else {
-      TSB_LAUNCH(TSB_POT_PLIFE)
-    }
-#undef TSB_LAUNCH
+    const bool vir = flags & (TSB_OUT_STRESS | TSB_OUT_STRESSES);
+    auto go = [&](auto pot_c) {
+      constexpr int POT = decltype(pot_c)::value;
+      auto run = [&](auto kernel) {
+        kernel(w, n, ns, table, nsp, cutoff, flags, forces, energies, stresses, active, st);
+      };
+      if (f64 && vir)
+        run(launch_forces<POT, double, P, true>);
+      else if (f64)
+        run(launch_forces<POT, double, P, false>);
+      else if (vir)
+        run(launch_forces<POT, float, P, true>);
+      else
+        run(launch_forces<POT, float, P, false>);
+    };
+    if (pot == TSB_POT_LJ)
+      go(std::integral_constant<int, TSB_POT_LJ>());
+    else if (pot == TSB_POT_MORSE)
+      go(std::integral_constant<int, TSB_POT_MORSE>());
+    else if (pot == TSB_POT_SOFT)
+      go(std::integral_constant<int, TSB_POT_SOFT>());
+    else
+      go(std::integral_constant<int, TSB_POT_PLIFE>());
   }
   k_sys_reduce<P><<<dim3((unsigned)ns, (unsigned)w.chunks), kBlock, 0, st>>>(
       w.b.geom, w.e_half, w.vir_half, flags, energy, stress, active, w.chunks, w.part);

@@ -38,7 +38,8 @@ __global__ void k_sys_reduce(const SysGeom *g, const double *e_half, const doubl
   for (int64_t a = lo + threadIdx.x; a < hi; a += blockDim.x) {
     int64_t i = G.start + a;
     acc[0] += e_half[i];
-    for (int k = 0; k < 6; ++k) acc[1 + k] += vir_half[6 * i + k];
+    if (flags & TSB_OUT_STRESS)
+      for (int k = 0; k < 6; ++k) acc[1 + k] += vir_half[6 * i + k];
   }
   for (int k = 0; k < 7; ++k) {
     for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
