@@ -373,6 +373,33 @@ int tsb_vv_kick(const double *p, const double *f, double half_dt, double *p_out,
                 int64_t n_atoms, void *stream);
 int tsb_adj_kick(double *lam_p, const double *lam_q, const double *inv_m, double dt,
                  int64_t n_atoms, void *stream);
+/* Whole trajectories and sweeps in one launch, one block per system (systems of at
+ * most tsb_adj_block_max_atoms() atoms, every periodic plane spacing >= cutoff +
+ * skin).  tsb_adj_trajectory: n_steps velocity-Verlet steps from (q, p); optional
+ * outputs: the state before every `every`-th step (ckpt_q / ckpt_p [.., N, 3]) and the
+ * positions before each step (traj [n_steps, N, 3]).  tsb_adj_sweep: the adjoint
+ * recursion back over traj (lam_q, lam_p in place, grad_params [S, ns, ns, 2] +=;
+ * `first`: traj starts at step 0, whose coefficient is dt / 2).  *status (int32, the
+ * caller's, zero before) becomes the neighbour count that exceeded max_neighbors, or
+ * 1 << 30 for a narrower cell; results are then meaningless.  TSB_ERR_CAPACITY: the
+ * lists do not fit a block's shared memory; TSB_ERR_UNSUPPORTED: too many atoms. */
+int tsb_adj_block_max_atoms(void);
+size_t tsb_adj_block_workspace_size(int64_t n_systems);
+int tsb_adj_trajectory(const double *table, int n_species, const int32_t *species,
+                       const double *cell_row, const uint8_t *pbc, const int64_t *system_idx,
+                       int64_t n_atoms, int64_t n_systems, int64_t max_system_atoms,
+                       double cutoff, double skin, int max_neighbors, const double *inv_m,
+                       const double *q, const double *p, double dt, int64_t n_steps,
+                       int64_t every, double *q_out, double *p_out, double *ckpt_q,
+                       double *ckpt_p, double *traj, int32_t *status, void *workspace,
+                       size_t workspace_bytes, void *stream);
+int tsb_adj_sweep(const double *table, int n_species, const int32_t *species,
+                  const double *cell_row, const uint8_t *pbc, const int64_t *system_idx,
+                  int64_t n_atoms, int64_t n_systems, int64_t max_system_atoms, double cutoff,
+                  double skin, int max_neighbors, const double *inv_m, const double *traj,
+                  double dt, int64_t n_steps, int first, double *lam_q, double *lam_p,
+                  double *grad_params, int32_t *status, void *workspace,
+                  size_t workspace_bytes, void *stream);
 int tsb_lj_hvp(const double *table, int n_species, const int32_t *species,
                const double *positions, const double *cell_row, const uint8_t *pbc,
                const int64_t *system_idx, int64_t n_atoms, int64_t n_systems, double cutoff,

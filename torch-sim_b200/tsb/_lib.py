@@ -58,6 +58,13 @@ PROTOTYPES = {
     "tsb_vv_kick_drift": (_int, [_vp, _vp, _vp, _vp, _dbl, _dbl, _vp, _vp, _i64, _vp]),
     "tsb_vv_kick": (_int, [_vp, _vp, _dbl, _vp, _i64, _vp]),
     "tsb_adj_kick": (_int, [_vp, _vp, _vp, _dbl, _i64, _vp]),
+    "tsb_adj_block_max_atoms": (_int, []),
+    "tsb_adj_block_workspace_size": (_sz, [_i64]),
+    "tsb_adj_trajectory": (_int, [_vp, _int, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _dbl, _dbl,
+                                  _int, _vp, _vp, _vp, _dbl, _i64, _i64, _vp, _vp, _vp, _vp,
+                                  _vp, _vp, _vp, _sz, _vp]),
+    "tsb_adj_sweep": (_int, [_vp, _int, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _dbl, _dbl, _int,
+                             _vp, _vp, _dbl, _i64, _int, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "tsb_lj_hvp": (_int, [_vp, _int, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _dbl, _vp, _dbl, _vp,
                           _vp, _i64, _vp, _sz, _vp]),
     "tsb_rdf_hist": (_int, [_vp, _vp, _vp, _vp, _i64, _i64, _dbl, _int, _dbl, _vp, _i64, _vp,

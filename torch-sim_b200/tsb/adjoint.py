@@ -142,6 +142,10 @@ class _ListOverflow(RuntimeError):
     pass
 
 
+class _NoBlocks(Exception):
+    """The problem does not fit the one-block-per-system kernels."""
+
+
 def _lists_fit(P, skin):
     """Every periodic plane spacing at least cutoff + skin (the lists' limit)."""
     inv = torch.linalg.inv(P.cell_row)
@@ -332,6 +336,115 @@ def _graphs_for(P: TrajectoryProblem, table: torch.Tensor) -> _Graphs:
     return G
 
 
+class _Blocks:
+    """Whole-trajectory launches, one block per system (``tsb_adj_trajectory`` /
+    ``tsb_adj_sweep``), for problems whose systems and lists fit a block: the list
+    capacity, grown from the device's report, and the calls.  Raises _NoBlocks when
+    they do not fit (too many atoms, a cell narrower than cutoff + skin, lists
+    beyond a block's shared memory); the caller then takes the graph path."""
+
+    SKIN = 1.0
+    CAP = 160            # neighbours per atom at first (argon at 9.5 A: ~100)
+    TRAJ_BYTES = 2 << 30  # positions of every step are kept up to this size
+
+    @staticmethod
+    def _common(P, table, cap, inv_m):
+        return (L.ptr(table), P.n_species, L.ptr(P.species), L.ptr(P.cell_row), L.ptr(P.pbc),
+                L.ptr(P.system_idx), P.n_atoms, P.n_systems, P.max_sys, P.cutoff,
+                _Blocks.SKIN, cap, L.ptr(inv_m))
+
+    @staticmethod
+    def run(P, body):
+        """``body(call)`` on this problem, again with longer lists
+        while the device reports an overflow (one read at the end)."""
+        lib, dev = L.load(), P.cell_row.device
+        if (P.max_sys > lib.tsb_adj_block_max_atoms() or P.n_species > 4
+                or P.cell_row.dtype != torch.float64):
+            raise _NoBlocks
+        ws = L.Workspace.get(dev, lib.tsb_adj_block_workspace_size(P.n_systems))
+        inv_m = (1.0 / P.masses).contiguous()
+        cap = P.__dict__.get("_block_cap", _Blocks.CAP)
+        while True:
+            status = torch.zeros(1, dtype=torch.int32, device=dev)
+
+            def call(name, table, *args):
+                try:
+                    L.call(name, *_Blocks._common(P, table, cap, inv_m), *args, L.ptr(status),
+                           L.ptr(ws), ws.numel(), L.stream_ptr(dev))
+                except L.TsbError as e:
+                    if e.status == L.TSB_ERR_CAPACITY:
+                        raise _NoBlocks from None
+                    raise
+
+            out = body(call)
+            needed = int(status.item())
+            if needed == 0:
+                P.__dict__["_block_cap"] = cap
+                return out
+            if needed >= (1 << 30):
+                raise _NoBlocks
+            cap = needed + needed // 8 + 4
+
+    @staticmethod
+    def _vec(t, P):
+        """[N, 3] FP64 on the problem's device."""
+        return torch.broadcast_to(t.to(P.cell_row), (P.n_atoms, 3)).contiguous()
+
+    @staticmethod
+    def trajectory(call, q, p, table, P, n_steps, ckpt=False, traj=None):
+        """(q_T, p_T, checkpoints {step: (q, p)}) after n_steps; ``traj`` gets the
+        positions before each step."""
+        every = P.checkpoint_every
+        qT, pT = torch.empty_like(q), torch.empty_like(p)
+        cq = cp = None
+        if ckpt:
+            cq = torch.empty((-(-n_steps // every), *q.shape), dtype=q.dtype, device=q.device)
+            cp = torch.empty_like(cq)
+        call("tsb_adj_trajectory", table, L.ptr(q), L.ptr(p), P.dt, n_steps, every, L.ptr(qT),
+             L.ptr(pT), L.ptr(cq), L.ptr(cp), L.ptr(traj))
+        return qT, pT, {k * every: (cq[k], cp[k]) for k in range(len(cq))} if ckpt else {}
+
+    @staticmethod
+    def sweep(call, traj, table, P, first, lam_q, lam_p, gpar):
+        call("tsb_adj_sweep", table, L.ptr(traj), P.dt, len(traj), int(first), L.ptr(lam_q),
+             L.ptr(lam_p), L.ptr(gpar))
+
+    @staticmethod
+    def integrate(q0, p0, table, P, keep_checkpoints):
+        q0, p0, table = _Blocks._vec(q0, P), _Blocks._vec(p0, P), table.contiguous()
+        return _Blocks.run(P, lambda call: _Blocks.trajectory(
+            call, q0, p0, table, P, P.n_steps, ckpt=keep_checkpoints))
+
+    @staticmethod
+    def loss_and_grad(table, q0, p0, P):
+        """(loss, lam_q, lam_p, gpar).  While every step's positions fit TRAJ_BYTES
+        they are kept and the sweep reads them; else each checkpoint segment is
+        integrated again before its sweep (memory O(N T / k + N k))."""
+        q0, p0, table = _Blocks._vec(q0, P), _Blocks._vec(p0, P), table.contiguous()
+        dev, f64, T = q0.device, torch.float64, P.n_steps
+        whole = 8 * q0.numel() * T <= _Blocks.TRAJ_BYTES
+        length = T if whole else min(P.checkpoint_every, T)
+        traj = torch.empty((length, *q0.shape), dtype=f64, device=dev)
+
+        def body(call):
+            qT, _, ckpt = _Blocks.trajectory(call, q0, p0, table, P, T, ckpt=not whole,
+                                             traj=traj if whole else None)
+            loss, h = loss_of(qT, P)
+            lam_q = _hist_grad(qT, 2.0 * (h - P.target), P)
+            lam_p = torch.zeros_like(lam_q)
+            gpar = torch.zeros((P.n_systems, P.n_species, P.n_species, 2), dtype=f64, device=dev)
+            if whole:
+                _Blocks.sweep(call, traj, table, P, True, lam_q, lam_p, gpar)
+            else:
+                for c in sorted(ckpt, reverse=True):
+                    seg = traj[:min(P.checkpoint_every, T - c)]
+                    _Blocks.trajectory(call, *ckpt[c], table, P, len(seg), traj=seg)
+                    _Blocks.sweep(call, seg, table, P, c == 0, lam_q, lam_p, gpar)
+            return loss, lam_q, lam_p, gpar
+
+        return _Blocks.run(P, body)
+
+
 def _retry_on_overflow(fn, P, table):
     """Run ``fn``; when a Verlet list overflowed, rebuild the graphs with a larger
     list and run it again."""
@@ -360,8 +473,13 @@ def _integrate_graphs(q0, p0, table, P, keep_checkpoints):
 def integrate(q0, p0, table, P: TrajectoryProblem, keep_checkpoints=True, use_graphs=True):
     """Velocity Verlet for ``P.n_steps`` steps from (q0, p0); returns (q_T, p_T, and
     the checkpoints {step: (q, p)} every ``P.checkpoint_every`` steps).  With
-    ``use_graphs`` each checkpoint segment replays one CUDA graph."""
+    ``use_graphs`` the trajectory is one launch (a block per system), or, where the
+    systems do not fit a block, each checkpoint segment replays one CUDA graph."""
     if use_graphs and q0.is_cuda and P.n_steps > 0:
+        try:
+            return _Blocks.integrate(q0, p0, table, P, keep_checkpoints)
+        except _NoBlocks:
+            pass
         return _retry_on_overflow(
             lambda: _integrate_graphs(q0, p0, table, P, keep_checkpoints), P, table)
     inv_m = (1.0 / P.masses).contiguous()
@@ -395,19 +513,29 @@ def _adjoint_graphs(table, ckpt, lam_q, P):
     return G.lam_q.clone(), G.lam_p.clone(), G.gpar.clone()
 
 
+def _fold(gpar):
+    """Gradients of sigma [ns,ns] and epsilon [ns,ns] from the per-system ones:
+    sigma_ab and sigma_ba are one parameter, so the gradient is symmetrised."""
+    g = gpar.sum(0)
+    return tuple(x + x.T - torch.diag(torch.diagonal(x)) for x in (g[..., 0], g[..., 1]))
+
+
 def loss_and_grad(sigma, epsilon, q0, p0, P: TrajectoryProblem, use_graphs=True):
     """Loss and its gradients w.r.t. sigma [ns,ns], epsilon [ns,ns], q0, p0."""
     table = lj_table(sigma, epsilon)
+    if use_graphs and q0.is_cuda and P.n_steps > 0:
+        try:
+            loss, lam_q, lam_p, gpar = _Blocks.loss_and_grad(table, q0, p0, P)
+            return (loss, *_fold(gpar), lam_q, lam_p)
+        except _NoBlocks:
+            pass
     qT, pT, ckpt = integrate(q0, p0, table, P, use_graphs=use_graphs)
     loss, h = loss_of(qT, P)
     lam_q = _hist_grad(qT, 2.0 * (h - P.target), P)
     if use_graphs and q0.is_cuda and P.n_steps > 0:
         lam_q, lam_p, gpar = _retry_on_overflow(
             lambda: _adjoint_graphs(table, ckpt, lam_q, P), P, table)
-        g = gpar.sum(0)
-        gs = g[..., 0] + g[..., 0].T - torch.diag(torch.diagonal(g[..., 0]))
-        ge = g[..., 1] + g[..., 1].T - torch.diag(torch.diagonal(g[..., 1]))
-        return loss, gs, ge, lam_q, lam_p
+        return (loss, *_fold(gpar), lam_q, lam_p)
     lam_p = torch.zeros_like(lam_q)
     gpar = torch.zeros((P.n_systems, P.n_species, P.n_species, 2), dtype=torch.float64,
                        device=q0.device)
@@ -424,11 +552,7 @@ def loss_and_grad(sigma, epsilon, q0, p0, P: TrajectoryProblem, use_graphs=True)
         for k in range(end - 1, c - 1, -1):
             _adj_kick(lam_p, lam_q, inv_m, P)
             _hvp(seg[k - c], table, lam_p, P.dt if k > 0 else P.dt / 2, lam_q, gpar, P)
-    g = gpar.sum(0)
-    # sigma_ab and sigma_ba are one parameter: symmetrise the gradient
-    gs = g[..., 0] + g[..., 0].T - torch.diag(torch.diagonal(g[..., 0]))
-    ge = g[..., 1] + g[..., 1].T - torch.diag(torch.diagonal(g[..., 1]))
-    return loss, gs, ge, lam_q, lam_p
+    return (loss, *_fold(gpar), lam_q, lam_p)
 
 
 class TrajectoryLoss(torch.autograd.Function):
