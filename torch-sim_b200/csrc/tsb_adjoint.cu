@@ -13,7 +13,7 @@
 // Also: the Gaussian-smeared pair-distance histogram of each system and its
 // gradient with respect to positions (the trajectory loss).
 #include "tsb_ljhvp.cuh"
-#include "tsb_search.cuh"
+#include "tsb_window.cuh"
 
 namespace tsb {
 
@@ -101,59 +101,87 @@ __device__ inline void rdf_window(double r, double bw, double width, int nb, int
   k1 = min(nb - 1, (int)floor((r + reach) / bw - 0.5));
 }
 
-__global__ void __launch_bounds__(128)
+// Both passes take one warp per atom over the gathered pairs (tsb_window.cuh).
+// (256 systems of 108 atoms: one thread per atom, each with ~60 pairs of ~10
+// exponentials one after another on 6 warps per SM, took 543 and 615 us; now 282 and
+// 126.)
+//
+// Histogram: a half-warp takes a pair, its lanes the pair's bins (lane = bin mod 16,
+// so no two lanes meet in a bin); the halves keep a histogram each in shared memory.
+// Beyond kRdfSmemBins bins the whole warp takes a pair, straight into the atom's row.
+constexpr int kRdfSmemBins = 128;
+
+__global__ void __launch_bounds__(32 * kWinWarps)
     k_rdf_part(BinData b, int64_t n, double r_max, int nb, double width, double *part) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ WinSmem win[kWinWarps];
+  __shared__ double hist[kWinWarps][2][kRdfSmemBins];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t p = (int64_t)blockIdx.x * kWinWarps + wid;
   if (p >= n) return;
   const double4 w = b.spos[p];
   const int i = tag_atom(w.w);
-  const SysGeom &G = b.geom[b.sys_of[i]];
-  double *h = part + (size_t)i * nb;
-  for (int k = 0; k < nb; ++k) h[k] = 0.0;
+  WinSmem &S = win[wid];
+  double *row = part + (size_t)i * nb;
+  const bool halves = nb <= kRdfSmemBins;
+  const int width_l = halves ? 16 : 32, side = lane / width_l, l = lane % width_l;
+  double *h = halves ? hist[wid][side] : row;
+  for (int k = l; k < nb; k += width_l) h[k] = 0.0;
   const double bw = r_max / nb, inv2w2 = 1.0 / (2.0 * width * width);
-  search_neighbors(G, b.spos, b.bin_start, i, w.x, w.y, w.z, r_max * r_max, false,
-                   [&](int, int, int, int, double, double, double, double d2) {
-                     const double r = sqrt(d2);
-                     int k0, k1;
-                     rdf_window(r, bw, width, nb, k0, k1);
-                     for (int k = k0; k <= k1; ++k) {
-                       const double x = r - (k + 0.5) * bw;
-                       h[k] += 0.5 * exp(-x * x * inv2w2);  // each pair is visited twice
-                     }
-                   });
+  window_gather(S, b.geom[b.sys_of[i]], b.spos, b.bin_start, w, r_max, [&](int kept) {
+    for (int t = side; t < kept; t += 32 / width_l) {
+      const double dx = S.x[t] - w.x, dy = S.y[t] - w.y, dz = S.z[t] - w.z;
+      const double d2 = dx * dx + dy * dy + dz * dz;
+      if (!(d2 < r_max * r_max) || (S.q[t] == p && (S.info[t] & 256))) continue;
+      const double r = sqrt(d2);
+      int k0, k1;
+      rdf_window(r, bw, width, nb, k0, k1);
+      for (int k = k0 + ((l - k0) & (width_l - 1)); k <= k1; k += width_l) {
+        const double x = r - (k + 0.5) * bw;
+        h[k] += 0.5 * exp(-x * x * inv2w2);  // each pair is visited twice
+      }
+    }
+  });
+  __syncwarp();
+  if (halves)
+    for (int k = lane; k < nb; k += 32) row[k] = hist[wid][0][k] + hist[wid][1][k];
 }
 
-// dL/dq_i = sum_j dL/dr_ij * (-u_ij), dL/dr = sum_b dL/dh_b * dg/dr
-__global__ void __launch_bounds__(128)
+// dL/dq_i = sum_j dL/dr_ij * (-u_ij), dL/dr = sum_b dL/dh_b * dg/dr: a lane per pair
+__global__ void __launch_bounds__(32 * kWinWarps)
     k_rdf_grad(BinData b, int64_t n, double r_max, int nb, double width,
                const double *__restrict__ dl_dh, double *__restrict__ grad) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ WinSmem win[kWinWarps];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t p = (int64_t)blockIdx.x * kWinWarps + wid;
   if (p >= n) return;
   const double4 w = b.spos[p];
   const int i = tag_atom(w.w);
   const int s = b.sys_of[i];
-  const SysGeom &G = b.geom[s];
+  WinSmem &S = win[wid];
   const double *dh = dl_dh + (size_t)s * nb;
   const double bw = r_max / nb, inv2w2 = 1.0 / (2.0 * width * width), iw2 = 1.0 / (width * width);
-  double gx = 0, gy = 0, gz = 0;
-  search_neighbors(G, b.spos, b.bin_start, i, w.x, w.y, w.z, r_max * r_max, false,
-                   [&](int, int, int, int, double dx, double dy, double dz, double d2) {
-                     const double r = sqrt(d2);
-                     double dlr = 0.0;
-                     int k0, k1;
-                     rdf_window(r, bw, width, nb, k0, k1);
-                     for (int k = k0; k <= k1; ++k) {
-                       const double x = r - (k + 0.5) * bw;
-                       dlr += dh[k] * (-x * iw2) * exp(-x * x * inv2w2);
-                     }
-                     const double ir = 1.0 / r;
-                     gx -= dlr * dx * ir;
-                     gy -= dlr * dy * ir;
-                     gz -= dlr * dz * ir;
-                   });
-  grad[3 * i] = gx;
-  grad[3 * i + 1] = gy;
-  grad[3 * i + 2] = gz;
+  double g[4] = {0.0, 0.0, 0.0, 0.0};
+  window_gather(S, b.geom[s], b.spos, b.bin_start, w, r_max, [&](int kept) {
+    for (int t = lane; t < kept; t += 32) {
+      const double dx = S.x[t] - w.x, dy = S.y[t] - w.y, dz = S.z[t] - w.z;
+      const double d2 = dx * dx + dy * dy + dz * dz;
+      if (!(d2 < r_max * r_max) || (S.q[t] == p && (S.info[t] & 256))) continue;
+      const double r = sqrt(d2);
+      double dlr = 0.0;
+      int k0, k1;
+      rdf_window(r, bw, width, nb, k0, k1);
+      for (int k = k0; k <= k1; ++k) {
+        const double x = r - (k + 0.5) * bw;
+        dlr += dh[k] * (-x * iw2) * exp(-x * x * inv2w2);
+      }
+      const double ir = 1.0 / r;
+      g[0] -= dlr * dx * ir;
+      g[1] -= dlr * dy * ir;
+      g[2] -= dlr * dz * ir;
+    }
+  });
+  const double t = warp_multi_sum<4>(g);
+  if (lane % 8 == 0 && lane < 24) grad[3 * (int64_t)i + lane / 8] = t;
 }
 
 // out[s, k] = sum over atoms of system s of part[i, k]  (fixed order)
@@ -285,7 +313,8 @@ extern "C" int tsb_rdf_hist(const double *positions, const double *cell_row, con
   cudaStream_t st = (cudaStream_t)stream;
   TSB_TRY(prepare_bins_any<double>(positions, cell_row, pbc, system_idx, n_atoms, n_systems,
                                    r_max, w.b, st, nullptr, max_system_atoms));
-  k_rdf_part<<<grid_for(n_atoms, 128), 128, 0, st>>>(w.b, n_atoms, r_max, n_bins, width, w.part);
+  k_rdf_part<<<grid_for(n_atoms, kWinWarps), 32 * kWinWarps, 0, st>>>(
+      w.b, n_atoms, r_max, n_bins, width, w.part);
   k_sum_parts<<<(unsigned)n_systems, 64, 0, st>>>(w.b.geom, w.part, n_bins, hist, 0);
   TSB_CHECK_LAUNCH();
   return TSB_OK;
@@ -307,7 +336,7 @@ extern "C" int tsb_rdf_hist_grad(const double *positions, const double *cell_row
   cudaStream_t st = (cudaStream_t)stream;
   TSB_TRY(prepare_bins_any<double>(positions, cell_row, pbc, system_idx, n_atoms, n_systems,
                                    r_max, w.b, st, nullptr, max_system_atoms));
-  k_rdf_grad<<<grid_for(n_atoms, 128), 128, 0, st>>>(w.b, n_atoms, r_max, n_bins, width,
+  k_rdf_grad<<<grid_for(n_atoms, kWinWarps), 32 * kWinWarps, 0, st>>>(w.b, n_atoms, r_max, n_bins, width,
                                                      dl_dhist, grad_positions);
   TSB_CHECK_LAUNCH();
   return TSB_OK;
