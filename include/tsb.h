@@ -152,7 +152,9 @@ int tsb_md_baoab_boa(void *positions, void *momenta, const void *forces,
  * (torch_sim/models/pair_potential.py:168-174); here the list holds all pairs
  * within cutoff + skin and is reused until an atom moved more than skin/2,
  * giving the same pairs and forces as PairPotentialModel.forward (:351-464).
- * tsb_verlet_build: cell-list search, ELL list[k * N + i] = j << 5 | image code,
+ * tsb_verlet_build: cell-list search, ELL list[k * N + i] = j << 5 | image code
+ *   (relative to the wrapped positions, or to FP32 positions as given where every
+ *   shift between those stays within one cell),
  *   counts [N], reference positions [N,3] f64, integer wraps [N,3] i32;
  *   *status > 0 if an atom had more than max_neighbors (regrow and rebuild);
  *   cell_row in `dtype`.

@@ -248,7 +248,9 @@ class VerletListModel(ModelInterface):
         self.n_builds += 1
         self._s_built = True
 
-    def _single_forward(self, state):
+    def _single_forward(self, state, energy=None, forces=None, stress=None):
+        """Results in the given contiguous buffers of the positions' dtype, or in new
+        ones."""
         if state.dtype != self._dtype:
             raise TypeError(f"SimState dtype {state.dtype} does not match model dtype "
                             f"{self._dtype}.")
@@ -265,10 +267,12 @@ class VerletListModel(ModelInterface):
                 self._s_build(state, pos)
                 self._s_check(state, pos, cell64)
         dt = pos.dtype
-        energy = torch.empty(1, dtype=dt, device=state.device)
-        forces = torch.empty_like(pos)
-        stress = (torch.empty((1, 3, 3), dtype=dt, device=state.device)
-                  if self._compute_stress else None)
+        energy = torch.empty(1, dtype=dt, device=state.device) if energy is None else energy
+        forces = torch.empty_like(pos) if forces is None else forces
+        if not self._compute_stress:
+            stress = None
+        elif stress is None:
+            stress = torch.empty((1, 3, 3), dtype=dt, device=state.device)
         flags = L.OUT_FORCES | (L.OUT_STRESS if stress is not None else 0)
         m = self.model
         L.call("tsb_verlet_forces", m.kind, L.ptr(m.table), m.n_species, L.ptr(self.s_list),
@@ -318,8 +322,16 @@ class VerletListModel(ModelInterface):
             if t is not None and not t.is_contiguous():
                 raise ValueError("forward_into needs contiguous output buffers")
         if sys_active is None and self._single_ok(state):
-            # one large system: its own kernels, results copied into the buffers
+            # one large system: its own kernels, writing into the buffers (or copied
+            # into ones of another dtype)
             self._last_single = True
+            shapes = ((energy, (1,)), (forces, tuple(state.positions.shape)),
+                      (stress, (1, 3, 3)))
+            if all(t is None or (t.dtype == state.positions.dtype and tuple(t.shape) == shape
+                                 and t.device == state.positions.device)
+                   for t, shape in shapes):
+                self._single_forward(state, energy, forces, stress)
+                return
             out = self._single_forward(state)
             energy.copy_(out["energy"])
             forces.copy_(out["forces"])
