@@ -192,9 +192,9 @@ __device__ __forceinline__ VerletSums verlet_sums(const POS *__restrict__ pos,
   // every entry and masked beyond the cutoff (no divergent branch)
   auto pair = [&](uint32_t e, const POS &wj) {
     const int code = (int)(e & 31u);
-    const double dx = (double)wj.x - xi + sv[3 * code];
-    const double dy = (double)wj.y - yi + sv[3 * code + 1];
-    const double dz = (double)wj.z - zi + sv[3 * code + 2];
+    const double dx = (double)wj.x - xi + sv[4 * code];
+    const double dy = (double)wj.y - yi + sv[4 * code + 1];
+    const double dz = (double)wj.z - zi + sv[4 * code + 2];
     const int sj = pos_species(wj);
     const double d2 = dx * dx + dy * dy + dz * dz;
     const bool in_ = d2 < rc2[sj];
@@ -262,9 +262,10 @@ __global__ void __launch_bounds__(256, 3)
                     const int32_t *__restrict__ cnt, int64_t n, const double *__restrict__ cell,
                     const double *__restrict__ table, int ns_species, double cutoff,
                     int flags, P *forces, double *part) {
-  __shared__ PairPrm<float> prm[kMaxSpecies * kMaxSpecies];
+  // (16-byte aligned rows and shifts are read in 16-byte pieces)
+  __shared__ alignas(16) PairPrm<float> prm[kMaxSpecies * kMaxSpecies];
   __shared__ double prc2[kMaxSpecies * kMaxSpecies];
-  __shared__ double sv[27 * 3];
+  __shared__ alignas(16) double sv[27 * 4];
   for (int k = threadIdx.x; k < ns_species * ns_species; k += blockDim.x) {
     prm[k] = make_prm<float>(POT, table + 5 * k, cutoff);
     prm_fast_extra(POT, table + 5 * k, prm[k]);
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(256, 3)
   }
   for (int k = threadIdx.x; k < 27; k += blockDim.x) {
     const int sx = k / 9 - 1, sy = (k / 3) % 3 - 1, sz = k % 3 - 1;
-    for (int m = 0; m < 3; ++m) sv[3 * k + m] = sx * cell[m] + sy * cell[3 + m] + sz * cell[6 + m];
+    for (int m = 0; m < 3; ++m) sv[4 * k + m] = sx * cell[m] + sy * cell[3 + m] + sz * cell[6 + m];
   }
   __syncthreads();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

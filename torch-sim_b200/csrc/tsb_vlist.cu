@@ -76,7 +76,7 @@ struct VlWork {
   int64_t *eoff;       // [S+1] their exclusive prefix (work list of the build)
   double4 *wpos;       // [N] current frame positions by slot, species in the high word
   float4 *wpos32;      // [N] the same in FP32, species bits in .w
-  float *svf;          // [81 S] FP32 shift vectors
+  float4 *svf;         // [27 S] FP32 shift vectors (one 16-byte read per entry)
   float *band;         // [S] FP32 decision band of r^2 (+inf: always FP64)
   double *sv;          // [81 S] S C per image code
   SysGeom *cur;        // [S] start / count / vol of the current cells
@@ -109,7 +109,7 @@ static void carve_vl(Carver &c, VlWork &w, int64_t n, int64_t ns) {
   w.eoff = c.take<int64_t>(ns + 1);
   w.wpos = c.take<double4>(n);
   w.wpos32 = c.take<float4>(n);
-  w.svf = c.take<float>(81 * ns);
+  w.svf = c.take<float4>(27 * ns);
   w.band = c.take<float>(ns);
   w.sv = c.take<double>(81 * ns);
   w.cur = c.take<SysGeom>(ns);
@@ -388,7 +388,7 @@ __global__ void k_vl_sys_built(const SysGeom *g, int64_t ns, int32_t *sys_exp, i
 template <class P>
 __global__ void k_vl_sys_geom(const P *cell_row, int64_t ns, const int64_t *lo,
                               const int64_t *hi, const double *rslack, double cutoff,
-                              double *sv, float *svf, float *band, SysGeom *cur) {
+                              double *sv, float4 *svf, float *band, SysGeom *cur) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 27 * ns) return;
   const int64_t s = t / 27;
@@ -396,11 +396,12 @@ __global__ void k_vl_sys_geom(const P *cell_row, int64_t ns, const int64_t *lo,
   double C[9];
   for (int k = 0; k < 9; ++k) C[k] = (double)cell_row[9 * s + k];
   const int sx = code / 9 - 1, sy = (code / 3) % 3 - 1, sz = code % 3 - 1;
+  double v[3];
   for (int m = 0; m < 3; ++m) {
-    const double v = sx * C[m] + sy * C[3 + m] + sz * C[6 + m];
-    sv[81 * s + 3 * code + m] = v;
-    svf[81 * s + 3 * code + m] = (float)v;
+    v[m] = sx * C[m] + sy * C[3 + m] + sz * C[6 + m];
+    sv[81 * s + 3 * code + m] = v[m];
   }
+  svf[27 * s + code] = make_float4((float)v[0], (float)v[1], (float)v[2], 0.0f);
   if (code) return;
   double bsum = 0.0;
   for (int k = 0; k < 3; ++k)
@@ -423,7 +424,7 @@ __global__ void k_vl_sys_geom(const P *cell_row, int64_t ns, const int64_t *lo,
 // current positions -> frame of the atom's build (FP64) by slot, species in .w
 template <class P>
 __global__ void k_vl_frame(const P *pos, const P *cell_row, const int64_t *sys,
-                           const int32_t *species, int64_t n, const int32_t *perm,
+                           const int32_t *species, int nsp, int64_t n, const int32_t *perm,
                            const int32_t *rwrap, double4 *wpos, float4 *wpos32) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
@@ -434,7 +435,8 @@ __global__ void k_vl_frame(const P *pos, const P *cell_row, const int64_t *sys,
   for (int m = 0; m < 3; ++m)
     w[m] = (double)pos[3 * i + m] -
            (W0 * (double)C[m] + W1 * (double)C[3 + m] + W2 * (double)C[6 + m]);
-  const unsigned long long hi = species ? (unsigned long long)(uint32_t)species[i] : 0ull;
+  // (a row of the table whatever the caller gave)
+  const unsigned long long hi = species ? (unsigned long long)min(max(species[i], 0), nsp - 1) : 0ull;
   wpos[p] = make_double4(w[0], w[1], w[2], __longlong_as_double((long long)(hi << 32)));
   wpos32[p] = make_float4((float)w[0], (float)w[1], (float)w[2], __int_as_float((int)hi));
 }
@@ -521,24 +523,26 @@ __global__ void __launch_bounds__(kVlBlock)
     k_vl_forces(const double4 *__restrict__ wpos, const float4 *__restrict__ wpos32,
                 const uint32_t *__restrict__ list, const int32_t *__restrict__ cnt, int64_t n,
                 const int32_t *__restrict__ perm, const int64_t *__restrict__ sys,
-                const double *__restrict__ sv, const float *__restrict__ svf,
+                const double *__restrict__ sv, const float4 *__restrict__ svf,
                 const float *__restrict__ band, const double *__restrict__ table,
                 int ns_species, double cutoff, int flags, P *forces, P *energies, P *stresses,
                 const SysGeom *__restrict__ cur, double *e_half, double *vir_half,
                 const uint8_t *__restrict__ active) {
   constexpr bool F32 = sizeof(R) == 4;
   using Pos4 = std::conditional_t<F32, float4, double4>;
-  using Sh = std::conditional_t<F32, float, double>;
-  __shared__ PairPrm<R> prm[kMaxSpecies * kMaxSpecies];
+  using Sh = std::conditional_t<F32, float4, double>;  // per shift: one, or three
+  constexpr int kSh = F32 ? 27 : 81;
+  // (16-byte aligned, so that a row and a shift are read in 16-byte pieces: with the
+  // species clamped once per call and the cutoff taken from the row, an entry costs
+  // XXX instructions instead of 91)
+  __shared__ alignas(16) PairPrm<R> prm[kMaxSpecies * kMaxSpecies];
   __shared__ double prc2[kMaxSpecies * kMaxSpecies];
-  __shared__ float prc2f[kMaxSpecies * kMaxSpecies];
-  __shared__ Sh ssv[kVlSmemSys * 81];
+  __shared__ alignas(16) Sh ssv[kVlSmemSys * kSh];
   __shared__ float sband[kVlSmemSys];
   for (int k = threadIdx.x; k < ns_species * ns_species; k += blockDim.x) {
     prm[k] = make_prm<R>(POT, table + 5 * k, cutoff);
     if constexpr (F32) prm_fast_extra(POT, table + 5 * k, prm[k]);
     prc2[k] = pair_rc2(POT, table + 5 * k, cutoff);
-    prc2f[k] = (float)prc2[k];
   }
   // slots are grouped by system, so a block spans systems s_lo..s_hi; the shift
   // vectors (FP32 ones and the bands on the FP32 path) of the first kVlSmemSys of
@@ -558,7 +562,7 @@ __global__ void __launch_bounds__(kVlBlock)
   const int64_t s_lo = sys[perm[p0]];
   const int64_t s_hi = sys[perm[min(p0 + (int64_t)(blockDim.x / LANES), n) - 1]];
   const int n_st = (int)min(s_hi - s_lo + 1, (int64_t)kVlSmemSys);
-  for (int k = threadIdx.x; k < 81 * n_st; k += blockDim.x) ssv[k] = shifts[81 * s_lo + k];
+  for (int k = threadIdx.x; k < kSh * n_st; k += blockDim.x) ssv[k] = shifts[kSh * s_lo + k];
   if constexpr (F32)
     for (int k = threadIdx.x; k < n_st; k += blockDim.x) sband[k] = band[s_lo + k];
   __syncthreads();
@@ -575,12 +579,11 @@ __global__ void __launch_bounds__(kVlBlock)
   }
   if (LANES == 1 && !valid) return;
   const Pos4 wi = wg[valid ? p : p0];
-  const int si = min(max(vl_species(wi.w), 0), ns_species - 1);
+  const int si = vl_species(wi.w);
   const PairPrm<R> *row = prm + si * ns_species;
   const double *rc2row = prc2 + si * ns_species;
-  const float *rc2frow = prc2f + si * ns_species;
   const bool staged = s - s_lo < n_st;
-  const Sh *svs = staged ? ssv + 81 * (s - s_lo) : shifts + 81 * s;
+  const Sh *svs = staged ? ssv + kSh * (s - s_lo) : shifts + kSh * s;
   float bnd = 0.f;
   if constexpr (F32) bnd = staged ? sband[s - s_lo] : band[s];
   const bool want_vir = flags & (TSB_OUT_STRESS | TSB_OUT_STRESSES);
@@ -594,20 +597,22 @@ __global__ void __launch_bounds__(kVlBlock)
 #define TSB_VLPAIR(E, WJ)                                                                    \
   {                                                                                          \
     const int code = (int)((E) & 31u);                                                       \
-    const int sj = min(max(vl_species((WJ).w), 0), ns_species - 1);                         \
+    const int sj = vl_species((WJ).w);                                                       \
+    const PairPrm<R> &pq = row[sj];                                                          \
     double dx, dy, dz;                                                                       \
     bool in_;                                                                                \
     R r2;                                                                                    \
     if constexpr (F32) {                                                                     \
-      const float ax = (WJ).x - wi.x + svs[3 * code];                                        \
-      const float ay = (WJ).y - wi.y + svs[3 * code + 1];                                    \
-      const float az = (WJ).z - wi.z + svs[3 * code + 2];                                    \
+      const float4 sh = svs[code];                                                           \
+      const float ax = (WJ).x - wi.x + sh.x;                                                 \
+      const float ay = (WJ).y - wi.y + sh.y;                                                 \
+      const float az = (WJ).z - wi.z + sh.z;                                                 \
       r2 = ax * ax + ay * ay + az * az;                                                      \
-      in_ = r2 < rc2frow[sj];                                                                \
+      in_ = r2 < pq.a3;                                                                      \
       dx = ax;                                                                               \
       dy = ay;                                                                               \
       dz = az;                                                                               \
-      if (!(fabsf(r2 - rc2frow[sj]) >= bnd)) {                                               \
+      if (!(fabsf(r2 - pq.a3) >= bnd)) {                                                     \
         const double4 di = wpos[p], dj = wpos[(E) >> 5];                                     \
         const double *sd = sv + 81 * s + 3 * code;                                           \
         dx = dj.x - di.x + sd[0];                                                            \
@@ -627,11 +632,11 @@ __global__ void __launch_bounds__(kVlBlock)
     if (F32 || in_) {                                                                        \
       R ep, fr;                                                                              \
       if constexpr (F32) {                                                                   \
-        pair_eval_fast<POT>(row[sj], r2, ep, fr);                                            \
+        pair_eval_fast<POT>(pq, r2, ep, fr);                                                 \
         fr = in_ ? fr : 0.f;                                                                 \
         ep = in_ ? ep : 0.f;                                                                 \
       } else {                                                                               \
-        pair_eval<POT, R>(row[sj], r2, ep, fr);                                              \
+        pair_eval<POT, R>(pq, r2, ep, fr);                                                   \
       }                                                                                      \
       const double gr = (double)fr;                                                          \
       const double gx = gr * dx, gy = gr * dy, gz = gr * dz;                                 \
@@ -799,7 +804,7 @@ static int vl_forces(int pot, const double *table, int nsp, const int32_t *speci
   k_vl_sys_geom<P><<<grid_for(27 * ns), kBlock, 0, st>>>(cell, ns, w.b.sys_lo, w.b.sys_hi,
                                                          w.rslack, cutoff, w.sv, w.svf, w.band,
                                                          w.cur);
-  k_vl_frame<P><<<grid_for(n), kBlock, 0, st>>>(pos, cell, sys, species, n, w.perm, w.rwrap,
+  k_vl_frame<P><<<grid_for(n), kBlock, 0, st>>>(pos, cell, sys, species, nsp, n, w.perm, w.rwrap,
                                                 w.wpos, w.wpos32);
   if (prune > 0.0) {
     // systems marked by the check or rebuilt since their last pruning form their
@@ -955,7 +960,8 @@ extern "C" int tsb_vlist_lj_hvp(const double *table, int n_species, const int32_
   k_vl_sys_geom<double><<<grid_for(27 * n_systems), kBlock, 0, st>>>(
       cell_row, n_systems, w.b.sys_lo, w.b.sys_hi, w.rslack, cutoff, w.sv, w.svf, w.band, w.cur);
   k_vl_frame<double><<<grid_for(n_atoms), kBlock, 0, st>>>(
-      positions, cell_row, system_idx, species, n_atoms, w.perm, w.rwrap, w.wpos, w.wpos32);
+      positions, cell_row, system_idx, species, n_species, n_atoms, w.perm, w.rwrap, w.wpos,
+      w.wpos32);
   k_vl_gather3<<<grid_for(3 * n_atoms), kBlock, 0, st>>>(v, w.perm, n_atoms, vs);
   if (n_atoms <= kGroupSearchMaxAtoms)
     k_vl_lj_hvp<kSearchGroup><<<grid_for(kSearchGroup * n_atoms, 128), 128, 0, st>>>(
