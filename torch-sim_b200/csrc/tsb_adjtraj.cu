@@ -492,13 +492,12 @@ static int blk_prepare(BlkSystem &B, const double *table, int nsp, const int32_t
     return TSB_ERR_INVALID_ARG;
   if (max_atoms > kBlkMaxAtoms) return TSB_ERR_UNSUPPORTED;
   Carver c(workspace, workspace_bytes);
-  int64_t *lo = c.take<int64_t>(ns), *hi = c.take<int64_t>(ns);
+  int64_t *lo = c.take<int64_t>(2 * ns), *hi = lo ? lo + ns : nullptr;
   if (!c.ok || !workspace) return TSB_ERR_WORKSPACE;
   const int stride = (int)(max_atoms + 1) / 2 * 2;
   if (blk_bytes((int)max_atoms, stride, cap, nsp, vecs) > (size_t)blk_smem_limit())
     return TSB_ERR_CAPACITY;
-  cudaMemsetAsync(lo, 0, sizeof(int64_t) * ns, st);
-  cudaMemsetAsync(hi, 0, sizeof(int64_t) * ns, st);
+  cudaMemsetAsync(lo, 0, 2 * sizeof(int64_t) * ns, st);  // and hi
   k_blk_bounds<<<grid_for(n), kBlock, 0, st>>>(system_idx, n, lo, hi);
   B = BlkSystem{table, nsp, species, cell, pbc, lo, hi, cutoff, skin, cap, stride, inv_m, dt,
                 status};

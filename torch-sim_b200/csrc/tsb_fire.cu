@@ -485,9 +485,10 @@ struct FireWork {
 };
 
 static void carve_fire(Carver &c, FireWork &w, int64_t ns) {
-  w.lo = c.take<int64_t>(ns);
-  w.hi = c.take<int64_t>(ns);
-  w.counter = c.take<int32_t>(4);
+  // (zeroed together by one memset)
+  w.lo = c.take<int64_t>(2 * ns + 2);
+  w.hi = w.lo ? w.lo + ns : nullptr;
+  w.counter = w.lo ? (int32_t *)(w.hi + ns) : nullptr;
   w.scr = c.take<double>(kFireScr * ns);
 }
 
@@ -502,9 +503,7 @@ static unsigned fire_probe_grid(int64_t n) {
 
 static int prep_bounds(FireWork &w, const int64_t *sys, int64_t n, int64_t ns,
                        cudaStream_t st) {
-  cudaMemsetAsync(w.lo, 0, sizeof(int64_t) * ns, st);
-  cudaMemsetAsync(w.hi, 0, sizeof(int64_t) * ns, st);
-  cudaMemsetAsync(w.counter, 0, sizeof(int32_t) * 4, st);
+  cudaMemsetAsync(w.lo, 0, sizeof(int64_t) * (2 * ns + 2), st);
   if (n > 0) k_bounds<<<grid_for(n), kBlock, 0, st>>>(sys, n, w.lo, w.hi);
   TSB_CHECK_LAUNCH();
   return TSB_OK;

@@ -251,6 +251,39 @@ __global__ void k_vl_exp_counts(const int32_t *sys_exp, const int64_t *lo, const
   if (s < ns) ecount[s] = sys_exp[s] ? (int32_t)(hi[s] - lo[s]) : 0;
 }
 
+// the same counts and their exclusive prefix in one block, for batches of at most
+// kVlOneScan systems: four passes of the block at most, where the counts and the scan
+// cost two to four launches of about 2 us each
+constexpr int64_t kVlOneScan = 4096;
+__global__ void __launch_bounds__(1024)
+    k_vl_exp_scan(const int32_t *sys_exp, const int64_t *lo, const int64_t *hi, int64_t ns,
+                  int64_t *eoff) {
+  __shared__ int64_t sums[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t carry = 0;
+  for (int64_t b0 = 0; b0 < ns; b0 += 1024) {
+    const int64_t s = b0 + threadIdx.x;
+    const int64_t v = s < ns && sys_exp[s] ? hi[s] - lo[s] : 0;
+    int64_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (lane == 31) sums[warp] = inc;
+    __syncthreads();
+    int64_t before = 0, total = 0;
+    for (int k = 0; k < 32; ++k) {
+      if (k < warp) before += sums[k];
+      total += sums[k];
+    }
+    if (s < ns) eoff[s] = carry + before + inc - v;
+    carry += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) eoff[ns] = carry;
+}
+
 // List search for the atoms of expired systems over fresh bins (cutoff + skin),
 // one warp per atom.  Work item t (< eoff[ns]) is atom t - eoff[s] of system s,
 // the last system with eoff[s] <= t (bisection; empty systems are skipped); a
@@ -392,10 +425,10 @@ __global__ void k_vl_sys_built(const SysGeom *g, int64_t ns, int32_t *sys_exp, i
 // per system for the force call: shift vectors (one thread per system and image
 // code), and from the code-0 thread the FP32 band, start / count and volume
 template <class P>
-__global__ void k_vl_sys_geom(const P *cell_row, int64_t ns, const int64_t *lo,
-                              const int64_t *hi, const double *rslack, double cutoff,
-                              double *sv, float4 *svf, float *band, SysGeom *cur) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ inline void vl_sys_geom(int64_t t, const P *cell_row, int64_t ns,
+                                   const int64_t *lo, const int64_t *hi, const double *rslack,
+                                   double cutoff, double *sv, float4 *svf, float *band,
+                                   SysGeom *cur) {
   if (t >= 27 * ns) return;
   const int64_t s = t / 27;
   const int code = (int)(t - 27 * s);
@@ -429,10 +462,10 @@ __global__ void k_vl_sys_geom(const P *cell_row, int64_t ns, const int64_t *lo,
 
 // current positions -> frame of the atom's build (FP64) by slot, species in .w
 template <class P>
-__global__ void k_vl_frame(const P *pos, const P *cell_row, const int64_t *sys,
-                           const int32_t *species, int nsp, int64_t n, const int32_t *perm,
-                           const int32_t *rwrap, double4 *wpos, float4 *wpos32) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ inline void vl_frame(int64_t p, const P *pos, const P *cell_row,
+                                const int64_t *sys, const int32_t *species, int nsp, int64_t n,
+                                const int32_t *perm, const int32_t *rwrap, double4 *wpos,
+                                float4 *wpos32) {
   if (p >= n) return;
   const int64_t i = perm[p];
   const P *C = cell_row + 9 * sys[i];
@@ -445,6 +478,28 @@ __global__ void k_vl_frame(const P *pos, const P *cell_row, const int64_t *sys,
   const unsigned long long hi = species ? (unsigned long long)min(max(species[i], 0), nsp - 1) : 0ull;
   wpos[p] = make_double4(w[0], w[1], w[2], __longlong_as_double((long long)(hi << 32)));
   wpos32[p] = make_float4((float)w[0], (float)w[1], (float)w[2], __int_as_float((int)hi));
+}
+
+// both, in one launch: the first blocks take the slots, the rest the systems
+template <class P>
+__global__ void k_vl_geom_frame(const P *pos, const P *cell_row, const int64_t *sys,
+                                const int32_t *species, int nsp, int64_t n, int64_t ns,
+                                unsigned frame_blocks, double cutoff, VlWork w) {
+  if (blockIdx.x < frame_blocks)
+    vl_frame<P>((int64_t)blockIdx.x * blockDim.x + threadIdx.x, pos, cell_row, sys, species, nsp,
+                n, w.perm, w.rwrap, w.wpos, w.wpos32);
+  else
+    vl_sys_geom<P>((int64_t)(blockIdx.x - frame_blocks) * blockDim.x + threadIdx.x, cell_row,
+                   ns, w.b.sys_lo, w.b.sys_hi, w.rslack, cutoff, w.sv, w.svf, w.band, w.cur);
+}
+
+template <class P>
+static void vl_geom_frame(const P *pos, const P *cell, const int64_t *sys,
+                          const int32_t *species, int nsp, int64_t n, int64_t ns, double cutoff,
+                          const VlWork &w, cudaStream_t st) {
+  const unsigned fb = grid_for(n);
+  k_vl_geom_frame<P><<<fb + grid_for(27 * ns), kBlock, 0, st>>>(pos, cell, sys, species, nsp, n,
+                                                               ns, fb, cutoff, w);
 }
 
 // Pruning of the systems marked in pexp: each slot's list is partitioned in
@@ -792,9 +847,13 @@ static int vl_build(const P *pos, const P *cell, const uint8_t *pbc, const int64
     TSB_TRY(prepare_bins_sys<P>(pos, cell, pbc, sys, n, ns, rcs, w.b, st, species, w.sys_exp));
   else
     TSB_TRY(prepare_bins<P>(pos, cell, pbc, sys, n, ns, rcs, w.b, st, species));
-  k_vl_exp_counts<<<grid_for(ns), kBlock, 0, st>>>(w.sys_exp, w.b.sys_lo, w.b.sys_hi, ns,
-                                                   w.ecount);
-  TSB_TRY(exclusive_scan(w.ecount, w.eoff, ns, w.b.scan_tmp, st));
+  if (ns <= kVlOneScan) {
+    k_vl_exp_scan<<<1, 1024, 0, st>>>(w.sys_exp, w.b.sys_lo, w.b.sys_hi, ns, w.eoff);
+  } else {
+    k_vl_exp_counts<<<grid_for(ns), kBlock, 0, st>>>(w.sys_exp, w.b.sys_lo, w.b.sys_hi, ns,
+                                                     w.ecount);
+    TSB_TRY(exclusive_scan(w.ecount, w.eoff, ns, w.b.scan_tmp, st));
+  }
   // a fixed grid of warps (8 blocks of 256 threads per SM) strides over the work
   int dev = 0, n_sm = 148;
   cudaGetDevice(&dev);
@@ -829,11 +888,7 @@ static int vl_forces(int pot, const double *table, int nsp, const int32_t *speci
                      const int64_t *sys, const uint8_t *active, int64_t n, int64_t ns,
                      double cutoff, double prune, int flags, P *energy, P *forces, P *stress,
                      P *energies, P *stresses, VlWork &w, cudaStream_t st) {
-  k_vl_sys_geom<P><<<grid_for(27 * ns), kBlock, 0, st>>>(cell, ns, w.b.sys_lo, w.b.sys_hi,
-                                                         w.rslack, cutoff, w.sv, w.svf, w.band,
-                                                         w.cur);
-  k_vl_frame<P><<<grid_for(n), kBlock, 0, st>>>(pos, cell, sys, species, nsp, n, w.perm, w.rwrap,
-                                                w.wpos, w.wpos32);
+  vl_geom_frame<P>(pos, cell, sys, species, nsp, n, ns, cutoff, w, st);
   if (prune > 0.0) {
     // systems marked by the check or rebuilt since their last pruning form their
     // front parts; the force kernel then reads the front counts
@@ -985,11 +1040,8 @@ extern "C" int tsb_vlist_lj_hvp(const double *table, int n_species, const int32_
   double *part = cs.take<double>(n_atoms * width);
   if (!cs.ok || !scratch) return TSB_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  k_vl_sys_geom<double><<<grid_for(27 * n_systems), kBlock, 0, st>>>(
-      cell_row, n_systems, w.b.sys_lo, w.b.sys_hi, w.rslack, cutoff, w.sv, w.svf, w.band, w.cur);
-  k_vl_frame<double><<<grid_for(n_atoms), kBlock, 0, st>>>(
-      positions, cell_row, system_idx, species, n_species, n_atoms, w.perm, w.rwrap, w.wpos,
-      w.wpos32);
+  vl_geom_frame<double>(positions, cell_row, system_idx, species, n_species, n_atoms, n_systems,
+                        cutoff, w, st);
   k_vl_gather3<<<grid_for(3 * n_atoms), kBlock, 0, st>>>(v, w.perm, n_atoms, vs);
   if (n_atoms <= kGroupSearchMaxAtoms)
     k_vl_lj_hvp<kSearchGroup><<<grid_for(kSearchGroup * n_atoms, 128), 128, 0, st>>>(
