@@ -330,6 +330,16 @@ int tsb_vlist_build(const void *positions, const void *cell_row, const uint8_t *
                     int64_t n_systems, int dtype, double cutoff, double skin, uint32_t *list,
                     int32_t *counts, int max_neighbors, int64_t max_system_atoms,
                     int32_t *flags, void *workspace, size_t workspace_bytes, void *stream);
+/* The same build with the pair table (rows as for tsb_vlist_forces): a pair is listed
+ * within its own cutoff + skin instead of the largest.  The forces then have to be
+ * taken with that table. */
+int tsb_vlist_build_pairs(int potential, const double *table, int n_species,
+                          const void *positions, const void *cell_row, const uint8_t *pbc,
+                          const int64_t *system_idx, const int32_t *species, int64_t n_atoms,
+                          int64_t n_systems, int dtype, double cutoff, double skin,
+                          uint32_t *list, int32_t *counts, int max_neighbors,
+                          int64_t max_system_atoms, int32_t *flags, void *workspace,
+                          size_t workspace_bytes, void *stream);
 /* tsb_vlist_lj_hvp: the adjoint's LJ Hessian-vector product (as tsb_lj_hvp:
  *   lam_q += coef * J_F(q)^T v, grad_params [S, ns, ns, 2] += coef *
  *   dF/d(sigma, epsilon)^T v) over lists built for `positions` (FP64; rows of

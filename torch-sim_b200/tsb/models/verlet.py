@@ -77,8 +77,11 @@ class VerletListModel(ModelInterface):
     def _ensure(self, state, pos, cell_row):
         n, ns = state.n_atoms, state.n_systems
         sysi, z = state.system_idx, state.atomic_numbers
+        # the species and the table's cutoffs decide which pairs are listed; the tensors
+        # are held below, so that no other one can come to lie at the same address
+        table = self.model.table
         key = (n, ns, pos.dtype, pos.device, sysi.data_ptr(), sysi._version, z.data_ptr(),
-               z._version)
+               z._version, table.data_ptr(), table._version)
         if self._key == key:
             return
         dev = pos.device
@@ -98,7 +101,7 @@ class VerletListModel(ModelInterface):
                               device=dev)
         self._reset(n, ns, dev)
         self._built = False
-        self._key = key
+        self._key, self._listed = key, (sysi, z, table)
 
     def _reset(self, n, ns, dev):
         L.call("tsb_vlist_reset", n, ns, L.ptr(self.ws), self.ws.numel(), L.stream_ptr(dev))
@@ -144,19 +147,24 @@ class VerletListModel(ModelInterface):
         return self._flags_host.tolist()
 
     # ---------------------------------------------------------------- lists
-    def _update_lists(self, state, pos, cell_row, pbc, sysi, species, active) -> bool:
+    def _update_lists(self, state, pos, cell_row, pbc, sysi, species, active,
+                      table) -> bool:
         """True when the flags are on their way and have to be read after the forces
         have been launched."""
         n, ns, dev = state.n_atoms, state.n_systems, pos.device
-        cutoff = self.model.cutoff
+        m, cutoff = self.model, self.model.cutoff
+
+        def build():
+            torch.ops.tsb.vlist_build_(pos, cell_row, pbc, sysi, species, ns, cutoff, self.skin,
+                                       self.list, self.counts, self.cap, self.max_system_atoms,
+                                       self.flags, self.ws, table, m.kind, m.n_species)
+
         if self.graph_safe:
             if self.sticky is None or self.sticky.device != dev:
                 self.sticky = torch.zeros(1, dtype=torch.int32, device=dev)
             torch.ops.tsb.vlist_check_(pos, cell_row, sysi, active, ns, cutoff, self.skin,
                                        self.prune, self.flags, self.ws)
-            torch.ops.tsb.vlist_build_(pos, cell_row, pbc, sysi, species, ns, cutoff, self.skin,
-                                       self.list, self.counts, self.cap, self.max_system_atoms,
-                                       self.flags, self.ws)
+            build()
             torch.maximum(self.sticky, self.flags[1:], out=self.sticky)
             return False
         if self._built:
@@ -165,9 +173,7 @@ class VerletListModel(ModelInterface):
             # marked; waiting left the GPU idle for ~0.06 ms in every step)
             torch.ops.tsb.vlist_check_(pos, cell_row, sysi, active, ns, cutoff, self.skin,
                                        self.prune, self.flags, self.ws)
-            torch.ops.tsb.vlist_build_(pos, cell_row, pbc, sysi, species, ns, cutoff, self.skin,
-                                       self.list, self.counts, self.cap, self.max_system_atoms,
-                                       self.flags, self.ws)
+            build()
             self._send_flags(self.flags)
             return True
         while True:
@@ -175,9 +181,7 @@ class VerletListModel(ModelInterface):
                                        self.prune, self.flags, self.ws)
             if not int(self.flags[0].item()):
                 break
-            torch.ops.tsb.vlist_build_(pos, cell_row, pbc, sysi, species, ns, cutoff, self.skin,
-                                       self.list, self.counts, self.cap, self.max_system_atoms,
-                                       self.flags, self.ws)
+            build()
             self.n_builds += 1
             st = int(self.flags[1].item())
             if st == 0:
@@ -207,10 +211,10 @@ class VerletListModel(ModelInterface):
         pbc = L.pbc_rows(state.pbc, n_sys, pos.device)
         sysi = state.system_idx.contiguous()
         species = self.model._species(state.atomic_numbers)
-        self._ensure(state, pos, cell_row)
-        pending = self._update_lists(state, pos, cell_row, pbc, sysi, species, active)
         m = self.model
         table = m.table if m.table.device == pos.device else m.table.to(pos.device)
+        self._ensure(state, pos, cell_row)
+        pending = self._update_lists(state, pos, cell_row, pbc, sysi, species, active, table)
         flags = 0
         if forces is not None:
             flags |= L.OUT_FORCES
@@ -236,7 +240,7 @@ class VerletListModel(ModelInterface):
         self.n_builds += 1 if marked else 0
         if overflow:
             self._grow_lists(overflow, state.n_atoms, n_sys, pos.device)
-            self._update_lists(state, pos, cell_row, pbc, sysi, species, active)
+            self._update_lists(state, pos, cell_row, pbc, sysi, species, active, table)
             evaluate()
 
     # ------------------------------------------------- one large system

@@ -289,18 +289,21 @@ _define("vlist_check_(Tensor positions, Tensor cell_row, Tensor system_idx, Tens
 
 
 def _vlist_build(positions, cell_row, pbc, system_idx, species, n_systems, cutoff, skin, lst,
-                 counts, max_neighbors, max_system_atoms, flags, workspace):
-    L.call("tsb_vlist_build", _P(positions), _P(cell_row), _P(pbc), _P(system_idx),
-           _P(species), positions.shape[0], int(n_systems), L.dtype_code(positions.dtype),
-           float(cutoff), float(skin), _P(lst), _P(counts), int(max_neighbors),
-           int(max_system_atoms), _P(flags), _P(workspace), workspace.numel(),
-           _stream(positions))
+                 counts, max_neighbors, max_system_atoms, flags, workspace, table=None, kind=0,
+                 n_species=1):
+    L.call("tsb_vlist_build_pairs", int(kind), _P(table), int(n_species), _P(positions),
+           _P(cell_row), _P(pbc), _P(system_idx), _P(species), positions.shape[0],
+           int(n_systems), L.dtype_code(positions.dtype), float(cutoff), float(skin), _P(lst),
+           _P(counts), int(max_neighbors), int(max_system_atoms), _P(flags), _P(workspace),
+           workspace.numel(), _stream(positions))
 
 
+# with the pair table each pair is listed within its own cutoff + skin
 _define("vlist_build_(Tensor positions, Tensor cell_row, Tensor pbc, Tensor system_idx, "
         "Tensor? species, int n_systems, float cutoff, float skin, Tensor(a!) nlist, "
         "Tensor(b!) counts, int max_neighbors, int max_system_atoms, Tensor(c!) flags, "
-        "Tensor(d!) workspace) -> ()", _vlist_build, _noop)
+        "Tensor(d!) workspace, Tensor? table=None, int kind=0, int n_species=1) -> ()",
+        _vlist_build, _noop)
 
 
 def _vlist_forces(kind, table, n_species, species, lst, counts, positions, cell_row,
