@@ -340,6 +340,9 @@ int tsb_vlist_build_pairs(int potential, const double *table, int n_species,
                           uint32_t *list, int32_t *counts, int max_neighbors,
                           int64_t max_system_atoms, int32_t *flags, void *workspace,
                           size_t workspace_bytes, void *stream);
+/* n <= 32 device flags into page-locked host memory, by a kernel: on the stream this
+ * costs a launch, where a copy costs some 20 us of waiting on either side. */
+int tsb_publish_flags(const int32_t *flags, int n, int32_t *host_flags, void *stream);
 /* tsb_vlist_lj_hvp: the adjoint's LJ Hessian-vector product (as tsb_lj_hvp:
  *   lam_q += coef * J_F(q)^T v, grad_params [S, ns, ns, 2] += coef *
  *   dF/d(sigma, epsilon)^T v) over lists built for `positions` (FP64; rows of

@@ -472,3 +472,21 @@ extern "C" int tsb_verlet_forces(int potential, const double *table, int n_speci
   TSB_CHECK_LAUNCH();
   return TSB_OK;
 }
+
+namespace tsb {
+// Flags straight into page-locked host memory.  The copy engine's turn for 8 bytes left
+// the stream idle for 10 to 20 us of every step (the kernel: 3.5 us; a step of 500,000
+// atoms 2598 -> 2520 us, 64 FIRE systems of 1024 atoms some 12 us a step).
+__global__ void k_publish_flags(const int32_t *flags, int n, volatile int32_t *host) {
+  if ((int)threadIdx.x < n) host[threadIdx.x] = flags[threadIdx.x];
+  __threadfence_system();
+}
+}  // namespace tsb
+
+extern "C" int tsb_publish_flags(const int32_t *flags, int n, int32_t *host_flags,
+                                 void *stream) {
+  if (!flags || !host_flags || n < 1 || n > 32) return TSB_ERR_INVALID_ARG;
+  k_publish_flags<<<1, 32, 0, (cudaStream_t)stream>>>(flags, n, host_flags);
+  TSB_CHECK_LAUNCH();
+  return TSB_OK;
+}

@@ -103,6 +103,7 @@ PROTOTYPES = {
                                _int, _i64, _vp, _vp, _sz, _vp]),
     "tsb_vlist_build_pairs": (_int, [_int, _vp, _int, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _int,
                                      _dbl, _dbl, _vp, _vp, _int, _i64, _vp, _vp, _sz, _vp]),
+    "tsb_publish_flags": (_int, [_vp, _int, _vp, _vp]),
     "tsb_vlist_hvp_scratch_size": (_sz, [_i64, _int]),
     "tsb_vlist_lj_hvp": (_int, [_vp, _int, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _dbl, _vp,
                                 _dbl, _vp, _vp, _vp, _sz, _vp, _sz, _vp]),

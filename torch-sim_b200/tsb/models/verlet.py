@@ -135,12 +135,14 @@ class VerletListModel(ModelInterface):
 
     # ---------------------------------------------------------------- flags
     def _send_flags(self, flags) -> None:
-        """Start copying device flags to pinned memory on the current stream."""
-        if self._flags_host is None or self._flags_host.numel() < flags.numel():
+        """Start writing device flags to pinned memory on the current stream."""
+        if self._flags_host is None:
             self._flags_host = torch.zeros(2, dtype=torch.int32).pin_memory()
-        self._flags_host[:flags.numel()].copy_(flags, non_blocking=True)
         self._flags_sent = torch.cuda.Event()
-        self._flags_sent.record(torch.cuda.current_stream(flags.device))
+        stream = torch.cuda.current_stream(flags.device)
+        L.call("tsb_publish_flags", L.ptr(flags), flags.numel(), L.ptr(self._flags_host),
+               stream.cuda_stream)
+        self._flags_sent.record(stream)
 
     def _read_flags(self) -> list[int]:
         self._flags_sent.synchronize()
@@ -233,10 +235,10 @@ class VerletListModel(ModelInterface):
                                         m.cutoff, self.prune, flags, energy, forces, stress,
                                         energies, stresses, self.ws)
 
-        evaluate()
-        if not pending:
-            return
-        marked, overflow = self._read_flags()
+        try:
+            evaluate()
+        finally:  # (the host buffer is in use until it has been read)
+            marked, overflow = self._read_flags() if pending else (0, 0)
         self.n_builds += 1 if marked else 0
         if overflow:
             self._grow_lists(overflow, state.n_atoms, n_sys, pos.device)
@@ -313,7 +315,9 @@ class VerletListModel(ModelInterface):
         L.require_cuda(state.positions, "state.positions")
         self._s_ensure(state)
         pos = state.positions.contiguous()
-        cell64 = state.cell[0].mT.double().contiguous()
+        # (one launch: type and layout in the same copy)
+        cell64 = torch.empty((3, 3), dtype=torch.float64, device=pos.device)
+        cell64.copy_(state.cell[0].mT)
         fresh = not self._s_built
         if fresh:
             self._s_build(state, pos)
@@ -337,8 +341,11 @@ class VerletListModel(ModelInterface):
                    L.ptr(stress), L.ptr(self.s_e_atom), L.ptr(self.s_vir_atom),
                    L.ptr(self.s_ws), self.s_ws.numel(), L.stream_ptr(state.device))
 
-        evaluate()
-        if not fresh and self._read_flags()[0]:
+        try:
+            evaluate()
+        finally:  # (the host buffer is in use until it has been read)
+            expired = not fresh and self._read_flags()[0]
+        if expired:
             self._s_build(state, pos)
             self._s_check(state, pos, cell64)
             evaluate()
