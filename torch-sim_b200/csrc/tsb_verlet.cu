@@ -475,8 +475,8 @@ extern "C" int tsb_verlet_forces(int potential, const double *table, int n_speci
 
 namespace tsb {
 // Flags straight into page-locked host memory.  The copy engine's turn for 8 bytes left
-// the stream idle for 10 to 20 us of every step (the kernel: 3.5 us; a step of 500,000
-// atoms 2598 -> 2520 us, 64 FIRE systems of 1024 atoms some 12 us a step).
+// the stream idle for 10 to 20 us of every step (the kernel: 3.5 us; ten steps of
+// 500,000 atoms 2612 -> 2525 us, 20 FIRE steps of 1024 Kob-Andersen systems 8017 -> 7903).
 __global__ void k_publish_flags(const int32_t *flags, int n, volatile int32_t *host) {
   if ((int)threadIdx.x < n) host[threadIdx.x] = flags[threadIdx.x];
   __threadfence_system();

@@ -299,8 +299,8 @@ __global__ void __launch_bounds__(1024)
 //
 // With the pair table, a pair is listed within its own cutoff + skin (reach2 of its
 // species) rather than the largest: the bound above holds for it all the more, and the
-// force kernel walks fewer entries that its own cutoffs would drop (64 Kob-Andersen
-// systems of 1024 atoms, skin 1.5 A: 245 -> 228 us per call).
+// force kernel walks fewer entries that its own cutoffs would drop (1024 Kob-Andersen
+// systems of 64 to 1000 atoms, skin 1.5 A: 245 -> 228 us per call).
 __global__ void __launch_bounds__(256, 4)
     k_vl_build(BinData b, int64_t n, int64_t ns, double cutoff, double skin, int pot,
                const double *__restrict__ table, int nsp, const int64_t *eoff, uint32_t *list,

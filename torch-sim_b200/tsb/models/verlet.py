@@ -35,6 +35,14 @@ from .pair_potential import PairTableModel
 
 
 class VerletListModel(ModelInterface):
+    # Batches of this many atoms have their lists rebuilt (the marked systems') without
+    # waiting for the check, smaller ones after reading its answer.  A FIRE step of Kob-
+    # Andersen systems, unread against read: 229 and 200 us at 6,000 atoms (the launches of
+    # a build that does nothing, with the host as the bound), 239 and 222 at 177,000, 290
+    # and 290 at 312,000, 343 and 363 at 422,000, 403 and 432 at 550,000 (the wait leaves
+    # the GPU idle).
+    UNREAD_ATOMS = 262144
+
     def __init__(self, model: PairTableModel, *, skin: float = 1.0, max_neighbors: int = 0,
                  prune: float | None = None):
         """``prune`` (Angstrom, batched lists only): between rebuilds each atom
@@ -134,15 +142,22 @@ class VerletListModel(ModelInterface):
             self.sticky.zero_()
 
     # ---------------------------------------------------------------- flags
-    def _send_flags(self, flags) -> None:
-        """Start writing device flags to pinned memory on the current stream."""
+    def _publish(self, flags):
+        """Device flags into pinned memory, on the current stream."""
         if self._flags_host is None:
             self._flags_host = torch.zeros(2, dtype=torch.int32).pin_memory()
-        self._flags_sent = torch.cuda.Event()
         stream = torch.cuda.current_stream(flags.device)
         L.call("tsb_publish_flags", L.ptr(flags), flags.numel(), L.ptr(self._flags_host),
                stream.cuda_stream)
-        self._flags_sent.record(stream)
+        return stream
+
+    def _flags_now(self, flags) -> list[int]:
+        self._publish(flags).synchronize()
+        return self._flags_host.tolist()
+
+    def _send_flags(self, flags) -> None:
+        self._flags_sent = torch.cuda.Event()
+        self._flags_sent.record(self._publish(flags))
 
     def _read_flags(self) -> list[int]:
         self._flags_sent.synchronize()
@@ -169,10 +184,8 @@ class VerletListModel(ModelInterface):
             build()
             torch.maximum(self.sticky, self.flags[1:], out=self.sticky)
             return False
-        if self._built:
-            # the rebuild touches only the systems that the check marked, so it is
-            # launched without waiting for the check's answer (0.02 ms when none is
-            # marked; waiting left the GPU idle for ~0.06 ms in every step)
+        if self._built and n >= self.UNREAD_ATOMS:
+            # (the rebuild touches only the systems that the check marked)
             torch.ops.tsb.vlist_check_(pos, cell_row, sysi, active, ns, cutoff, self.skin,
                                        self.prune, self.flags, self.ws)
             build()
@@ -181,7 +194,7 @@ class VerletListModel(ModelInterface):
         while True:
             torch.ops.tsb.vlist_check_(pos, cell_row, sysi, active, ns, cutoff, self.skin,
                                        self.prune, self.flags, self.ws)
-            if not int(self.flags[0].item()):
+            if not self._flags_now(self.flags)[0]:
                 break
             build()
             self.n_builds += 1
