@@ -25,7 +25,7 @@
 // One thread per atom, which this replaces, issued about five times the instructions:
 // the lanes of a warp walked bins of different lengths, each bin a bounds load and
 // image arithmetic for ~2 atoms.  Measured against it (B200): forces of 540,000
-// copper atoms, FP32, 1292 -> 545 us; of 548,000 Kob-Andersen atoms, FP64 with
+// copper atoms, FP32, 1292 -> 604 us; of 548,000 Kob-Andersen atoms, FP64 with
 // stress, 1430 -> 728 us; counting the pairs of 500,000 argon atoms 692 -> 208 us.
 // Tried and dropped: one warp per bin (945 us for the argon count: the gathering is
 // paid per bin, and 2 atoms share it), one block of four warps per 2 x 2 x 2 bins
