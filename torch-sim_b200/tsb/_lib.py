@@ -52,6 +52,7 @@ PROTOTYPES = {
                                 _vp]),
     "tsb_md_kick": (_int, [_vp, _vp, _vp, _vp, _dbl, _i64, _int, _vp]),
     "tsb_md_drift": (_int, [_vp, _vp, _vp, _vp, _vp, _dbl, _i64, _int, _vp]),
+    "tsb_md_kick_drift": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _dbl, _dbl, _i64, _int, _vp]),
     "tsb_md_baoab_boa": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _u64, _u64,
                                 _vp, _i64, _int, _vp]),
     "tsb_adjoint_workspace_size": (_sz, [_i64, _i64, _i64]),

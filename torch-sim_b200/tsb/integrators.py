@@ -120,9 +120,10 @@ def _kick(state, dt_s, scale):
     torch.ops.tsb.md_kick_(state.momenta, state.forces, state.system_idx, dt_s, float(scale))
 
 
-def _drift(state, dt_s, scale):
-    torch.ops.tsb.md_drift_(state.positions, state.momenta, state.masses, state.system_idx,
-                            dt_s, float(scale))
+def _kick_drift(state, dt_s):
+    """B(dt/2) A(dt)"""
+    torch.ops.tsb.md_kick_drift_(state.positions, state.momenta, state.forces, state.masses,
+                                 state.system_idx, dt_s, 0.5, 1.0)
 
 
 def use_device_counter(state, counter_dev: torch.Tensor | None = None):
@@ -175,8 +176,7 @@ def nve_step(state, model, *, dt, **_kw):
     """B(dt/2) A(dt) force B(dt/2) (nve.py:74-130)."""
     _prepare(state)
     dt_s = _per_system(dt, state.n_systems, state.device)
-    _kick(state, dt_s, 0.5)
-    _drift(state, dt_s, 1.0)
+    _kick_drift(state, dt_s)
     _update_forces(state, model)
     _kick(state, dt_s, 0.5)
     return state
@@ -294,8 +294,7 @@ def nvt_nose_hoover_step(state, model, *, dt, kT, **_kw):
     dt_s = _per_system(dt, state.n_systems, state.device)
     kT_s = _per_system(kT, state.n_systems, state.device)
     _nhc_half(state, kT_s, recompute=False)
-    _kick(state, dt_s, 0.5)
-    _drift(state, dt_s, 1.0)
+    _kick_drift(state, dt_s)
     _update_forces(state, model)
     _kick(state, dt_s, 0.5)
     _nhc_half(state, kT_s, recompute=True)
@@ -347,8 +346,7 @@ def nvt_vrescale_step(model, state, *, dt, kT, tau=None, noise=None, **_kw):
            L.ptr(tau_s), L.ptr(dt_s), L.ptr(noise), seed & (2**64 - 1), counter, None,
            L.ptr(ws), ws.numel(), L.stream_ptr(dev))
     state._philox_seed, state._philox_counter = seed, counter + 1
-    _kick(state, dt_s, 0.5)
-    _drift(state, dt_s, 1.0)
+    _kick_drift(state, dt_s)
     _update_forces(state, model)
     _kick(state, dt_s, 0.5)
     return state

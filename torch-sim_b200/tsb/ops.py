@@ -177,6 +177,16 @@ _define("md_drift_(Tensor(a!) positions, Tensor momenta, Tensor masses, Tensor s
         "Tensor dt, float scale) -> ()", _md_drift, _noop)
 
 
+def _md_kick_drift(positions, momenta, forces, masses, system_idx, dt, kick, drift):
+    L.call("tsb_md_kick_drift", _P(positions), _P(momenta), _P(forces), _P(masses),
+           _P(system_idx), _P(dt), float(kick), float(drift), positions.shape[0],
+           L.dtype_code(positions.dtype), _stream(positions))
+
+
+_define("md_kick_drift_(Tensor(a!) positions, Tensor(b!) momenta, Tensor forces, Tensor masses, "
+        "Tensor system_idx, Tensor dt, float kick, float drift) -> ()", _md_kick_drift, _noop)
+
+
 def _md_baoab_boa(positions, momenta, forces, masses, system_idx, dt, kT, gamma, noise, seed,
                   counter, counter_dev):
     L.call("tsb_md_baoab_boa", _P(positions), _P(momenta), _P(forces), _P(masses),
@@ -326,7 +336,7 @@ _define("vlist_forces_(int kind, Tensor table, int n_species, Tensor? species, "
         _vlist_forces, _noop)
 
 
-OPS = ("nl_build", "pair_forward", "pair_forward_into_", "md_kick_", "md_drift_",
+OPS = ("nl_build", "pair_forward", "pair_forward_into_", "md_kick_", "md_drift_", "md_kick_drift_",
        "md_baoab_boa_", "fused_md_", "fire_ase_pre_", "fire_vv_pre_", "fire_vv_post_",
        "frechet_cell_forces_", "fire_converged_", "vlist_check_", "vlist_build_",
        "vlist_forces_")
