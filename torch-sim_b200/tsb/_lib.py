@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import threading
+import weakref
 
 import torch
 
@@ -200,23 +201,26 @@ def call(name: str, *args):
     return st
 
 
-_MAX_SYS_CACHE: dict = {}
+_MAX_SYS: dict = {}  # id of a tensor -> (weak reference, version, length, systems, value)
 
 
 def max_system_atoms(system_idx: torch.Tensor, n_systems: int) -> int:
-    """Largest system's atom count (the binning hint of the C ABI), cached per
-    system_idx tensor version (one device read when it changes)."""
-    key = (system_idx.data_ptr(), system_idx._version, system_idx.shape[0], n_systems)
-    hit = _MAX_SYS_CACHE.get(key)
-    if hit is None:
-        if system_idx.numel() == 0:
-            hit = 0
-        else:
-            hit = int(torch.bincount(system_idx, minlength=n_systems).max())
-        if len(_MAX_SYS_CACHE) > 64:
-            _MAX_SYS_CACHE.clear()
-        _MAX_SYS_CACHE[key] = hit
-    return hit
+    """Largest system's atom count, kept for a tensor as long as it lives and is not
+    written to (one device read when it changes).  The entry belongs to the tensor
+    itself: an address says nothing once its tensor is gone and another lies there."""
+    key = id(system_idx)
+    now = (system_idx._version, system_idx.shape[0], n_systems)
+    hit = _MAX_SYS.get(key)
+    if hit is not None and hit[0]() is system_idx and hit[1:4] == now:
+        return hit[4]
+    value = int(torch.bincount(system_idx, minlength=n_systems).max()) if now[1] else 0
+
+    def forget(ref):
+        if key in _MAX_SYS and _MAX_SYS[key][0] is ref:
+            del _MAX_SYS[key]
+
+    _MAX_SYS[key] = (weakref.ref(system_idx, forget), *now, value)
+    return value
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
