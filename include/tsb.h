@@ -400,7 +400,9 @@ int tsb_adj_kick(double *lam_p, const double *lam_q, const double *inv_m, double
  * recursion back over traj (lam_q, lam_p in place, grad_params [S, ns, ns, 2] +=;
  * `first`: traj starts at step 0, whose coefficient is dt / 2).  *status (int32, the
  * caller's, zero before) becomes the neighbour count that exceeded max_neighbors, or
- * 1 << 30 for a narrower cell; results are then meaningless.  TSB_ERR_CAPACITY: the
+ * 1 << 30 for a narrower cell or a system of more than max_system_atoms atoms; the
+ * results of such systems are then meaningless.  max_system_atoms sizes the blocks: it
+ * may be larger than the largest system, and a larger system is left out whole.  TSB_ERR_CAPACITY: the
  * lists do not fit a block's shared memory; TSB_ERR_UNSUPPORTED: too many atoms. */
 int tsb_adj_block_max_atoms(void);
 size_t tsb_adj_block_workspace_size(int64_t n_systems);

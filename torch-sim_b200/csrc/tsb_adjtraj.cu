@@ -17,8 +17,9 @@
 // Lists.  Entry: neighbour | image code << 11, image S in {-1,0,1}^3 of the build's
 // wrapped positions, within cutoff + skin; every thread of a block agrees to rebuild
 // when an atom moved more than skin / 2 since the build (the barrier carries the
-// vote).  Needs every periodic plane spacing >= cutoff + skin; a narrower cell or a
-// full list is reported in `status` and the caller takes the general path.
+// vote).  Needs every periodic plane spacing >= cutoff + skin; a narrower cell, a
+// full list or a system larger than the caller said is reported in `status` and the
+// caller takes the general path.
 #include "tsb_common.cuh"
 #include "tsb_search.cuh"
 
@@ -116,9 +117,14 @@ struct BlkThread {
   bool on;           // has an atom
   int64_t i;         // ... its index
 
-  // whole block, barriers inside; false (for every thread) without lists
-  __device__ bool setup(const BlkSystem &B, BlkSmem &S, int64_t s) {
+  // whole block, barriers inside; false (for every thread) without lists.  A system of
+  // more atoms than the block was sized for is reported before anything of it is touched.
+  __device__ bool setup(const BlkSystem &B, BlkSmem &S, int64_t s, int max_atoms) {
     const int64_t lo = B.lo[s];
+    if (B.hi[s] - lo > max_atoms) {
+      if (threadIdx.x == 0) atomicMax(B.status, 1 << 30);
+      return false;
+    }
     n = (int)(B.hi[s] - lo);
     a = threadIdx.x / LANES;
     lane = threadIdx.x % LANES;
@@ -303,7 +309,7 @@ __global__ void __launch_bounds__(kBlkThreads, 2)
   BlkSmem S = blk_carve(smem, max_atoms, B.stride, B.cap, B.nsp, 0);
   BlkThread<LANES> t;
   blk_table(B, S);
-  if (!t.setup(B, S, blockIdx.x)) return;  // (the same for every thread)
+  if (!t.setup(B, S, blockIdx.x, max_atoms)) return;  // (the same for every thread)
   const bool lead = t.on && t.lane == 0;
   double q[3], p[3], f[3], im = 0.0;
   for (int m = 0; m < 3; ++m) {
@@ -360,7 +366,7 @@ __global__ void __launch_bounds__(kBlkThreads, NS <= 2 ? 2 : 1)
   BlkSmem S = blk_carve(smem, max_atoms, B.stride, B.cap, B.nsp, 1);
   BlkThread<LANES> t;
   blk_table(B, S);
-  if (!t.setup(B, S, blockIdx.x)) return;
+  if (!t.setup(B, S, blockIdx.x, max_atoms)) return;
   const bool lead = t.on && t.lane == 0;
   if (lead) {
     S.lx[t.a] = lam_q[3 * t.i];
