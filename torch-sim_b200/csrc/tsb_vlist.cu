@@ -614,6 +614,23 @@ __global__ void __launch_bounds__(kVlBlock)
   __shared__ alignas(16) Sh ssv[kVlSmemSys * kSh];
   __shared__ float sband[kVlSmemSys];
   __shared__ float4 near_pos[F32 ? kVlStage : 1];
+  // LANES lanes per slot (small batches: more threads in flight; each lane takes
+  // every LANES-th entry and a fixed butterfly sums the lanes), else one thread
+  const int64_t p0 = (int64_t)blockIdx.x * (blockDim.x / LANES);
+  const int64_t p1 = min(p0 + (int64_t)(blockDim.x / LANES), n);
+  const int64_t p = p0 + threadIdx.x / LANES;
+  const int lane = threadIdx.x % LANES;
+  // a group whose slot is past the end or inactive still takes part in the
+  // lane sums (with no entries) and leaves before writing
+  bool valid = p < n;
+  int64_t i = 0, s = 0;
+  if (valid) {
+    i = perm[p];
+    s = sys[i];
+    valid = !active || active[s];
+  }
+  // (a block of frozen systems, which may never have had lists, reads nothing of them)
+  if (active && !__syncthreads_or(valid)) return;
   for (int k = threadIdx.x; k < ns_species * ns_species; k += blockDim.x) {
     prm[k] = make_prm<R>(POT, table + 5 * k, cutoff);
     if constexpr (F32) prm_fast_extra(POT, table + 5 * k, prm[k]);
@@ -631,44 +648,31 @@ __global__ void __launch_bounds__(kVlBlock)
     shifts = sv;
     wg = wpos;
   }
-  // LANES lanes per slot (small batches: more threads in flight; each lane takes
-  // every LANES-th entry and a fixed butterfly sums the lanes), else one thread
-  const int64_t p0 = (int64_t)blockIdx.x * (blockDim.x / LANES);
   const int64_t s_lo = sys[perm[p0]];
-  const int64_t s_hi = sys[perm[min(p0 + (int64_t)(blockDim.x / LANES), n) - 1]];
-  const int n_st = (int)min(s_hi - s_lo + 1, (int64_t)kVlSmemSys);
+  const int64_t s_hi = sys[perm[p1 - 1]];
+  const int n_st = (int)max(min(s_hi - s_lo + 1, (int64_t)kVlSmemSys), (int64_t)0);
   for (int k = threadIdx.x; k < kSh * n_st; k += blockDim.x) ssv[k] = shifts[kSh * s_lo + k];
   if constexpr (F32)
     for (int k = threadIdx.x; k < n_st; k += blockDim.x) sband[k] = band[s_lo + k];
-  // every neighbour lies in one of those systems: their FP32 positions (16 KB per
-  // thousand atoms) are staged as well where they fit
+  // every neighbour lies in one of the block's systems, which lie side by side in the
+  // slots whatever their numbers: their FP32 positions (16 KB per thousand atoms) are
+  // staged as well where they fit
   bool near_ = false;
   int64_t g0 = 0;
   if constexpr (F32) {
     g0 = cur[s_lo].start;
     const int64_t g1 = cur[s_hi].start + cur[s_hi].count;
-    near_ = g1 - g0 <= kVlStage;
+    near_ = 0 <= g0 && g0 <= p0 && p1 <= g1 && g1 <= n && g1 - g0 <= kVlStage;
     if (near_)
       for (int k = threadIdx.x; k < (int)(g1 - g0); k += blockDim.x) near_pos[k] = wpos32[g0 + k];
   }
   __syncthreads();
-  const int64_t p = p0 + threadIdx.x / LANES;
-  const int lane = threadIdx.x % LANES;
-  // a group whose slot is past the end or inactive still takes part in the
-  // lane sums (with no entries) and leaves before writing
-  bool valid = p < n;
-  int64_t i = 0, s = s_lo;
-  if (valid) {
-    i = perm[p];
-    s = sys[i];
-    valid = !active || active[s];
-  }
   if (LANES == 1 && !valid) return;
   const Pos4 wi = wg[valid ? p : p0];
   const int si = vl_species(wi.w);
   const PairPrm<R> *row = prm + si * ns_species;
   const double *rc2row = prc2 + si * ns_species;
-  const bool staged = s - s_lo < n_st;
+  const bool staged = s >= s_lo && s - s_lo < n_st;
   const Sh *svs = staged ? ssv + kSh * (s - s_lo) : shifts + kSh * s;
   float bnd = 0.f;
   if constexpr (F32) bnd = staged ? sband[s - s_lo] : band[s];
@@ -1089,6 +1093,7 @@ extern "C" int tsb_vlist_reset(int64_t n_atoms, int64_t n_systems, void *workspa
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(w.sys_built, 0, sizeof(int32_t) * n_systems, st);
   cudaMemsetAsync(w.sys_exp, 0, sizeof(int32_t) * n_systems, st);
+  cudaMemsetAsync(w.b.sys_lo, 0, 2 * sizeof(int64_t) * n_systems, st);  // and sys_hi
   cudaMemsetAsync(w.rslack, 0xff, sizeof(double) * n_systems, st);  // NaN: FP64 test
   cudaMemsetAsync(w.pexp, 0xff, sizeof(int32_t) * n_systems, st);    // nonzero: prune
   k_vl_iota<<<grid_for(n_atoms), kBlock, 0, st>>>(w.perm, n_atoms);
