@@ -47,3 +47,53 @@ def test_nothing_is_kept_of_a_tensor_that_is_gone():
         L.max_system_atoms(torch.zeros(n, dtype=torch.int64), 1)
     gc.collect()
     assert len(L._MAX_SYS) <= before
+
+
+def test_species_of_other_atoms_at_an_old_address():
+    from tsb import models
+
+    model = models.kob_andersen_model(device="cpu")
+    for _ in range(50):
+        a = torch.tensor([1, 1, 2, 2] * 100)
+        at = a.data_ptr()
+        assert torch.equal(model._species(a), (a - 1).int())
+        del a
+        b = torch.tensor([2, 1, 2, 1] * 100)
+        assert torch.equal(model._species(b), (b - 1).int())
+        if b.data_ptr() == at:
+            break
+
+
+def test_order_of_other_systems_at_an_old_address():
+    from tsb import integrators
+
+    class State:
+        pass
+
+    st = State()
+    for _ in range(50):
+        st.system_idx, st.n_atoms, st.n_systems = torch.tensor([0] * 300 + [1] * 20), 320, 2
+        at = st.system_idx.data_ptr()
+        assert integrators._system_order(st)[0].tolist() == [0, 1]
+        st.system_idx = None
+        st.system_idx = torch.tensor([0] * 20 + [1] * 300)
+        order, most = integrators._system_order(st)
+        assert order.tolist() == [1, 0] and most == 300
+        if st.system_idx.data_ptr() == at:
+            break
+    st.system_idx[20:] = 0  # written to in place
+    assert integrators._system_order(st)[1] == 320
+
+
+def test_what_counts_as_the_same_tensor():
+    import copy
+    import pickle
+
+    a = torch.arange(12)
+    seen = L.Seen(a)
+    assert seen.same(a) and seen.same(a.view(12)) and not seen.same(a.clone())
+    assert not seen.same(a[:6]) and not seen.same(a.view(3, 4))
+    assert not L.Seen(a[:6]).same(a[::2])  # one address, one length
+    assert not copy.deepcopy(seen).same(a) and not pickle.loads(pickle.dumps(seen)).same(a)
+    a[0] = 5
+    assert not seen.same(a) and not L.Seen().same(a)

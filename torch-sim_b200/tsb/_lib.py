@@ -223,6 +223,28 @@ def max_system_atoms(system_idx: torch.Tensor, n_systems: int) -> int:
     return value
 
 
+class Seen:
+    """A tensor that something was worked out for.  The tensor is held, so its memory is
+    not handed to another one meanwhile: what has its address and shape is the same data,
+    written to or not (``_version``).  A copy (``copy.deepcopy``, pickling) has seen
+    nothing."""
+
+    def __init__(self, t: torch.Tensor | None = None):
+        self.t, self.version = t, None if t is None else t._version
+
+    def __reduce__(self):
+        return Seen, ()
+
+    def __deepcopy__(self, _memo):
+        return Seen()
+
+    def same(self, t: torch.Tensor) -> bool:
+        s = self.t
+        return s is not None and self.version == t._version and (s is t or (
+            s.data_ptr() == t.data_ptr() and s.shape == t.shape and s.dtype == t.dtype
+            and s.stride() == t.stride() and s.device == t.device))
+
+
 def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 

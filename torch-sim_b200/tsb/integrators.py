@@ -828,14 +828,13 @@ class FusedMDError(RuntimeError):
 def _system_order(state):
     """Largest systems first (longest-processing-time order balances the tail)."""
     cache = getattr(state, "_tsb_order", None)
-    key = (state.system_idx.data_ptr(), state.n_atoms)
-    if cache is not None and cache[0] == key:
+    if cache is not None and cache[0].same(state.system_idx):
         return cache[1], cache[2]
     counts = torch.bincount(state.system_idx, minlength=state.n_systems)
     order = torch.argsort(counts, descending=True, stable=True).to(torch.int32).contiguous()
     max_atoms = int(counts.max())
     try:
-        state._tsb_order = (key, order, max_atoms)
+        state._tsb_order = (L.Seen(state.system_idx), order, max_atoms)
     except AttributeError:
         pass
     return order, max_atoms

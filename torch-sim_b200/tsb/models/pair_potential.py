@@ -85,13 +85,12 @@ class PairTableModel(ModelInterface):
             lut = torch.full((int(z.max()) + 1,), -1, dtype=torch.int32)
             lut[z] = torch.arange(len(z), dtype=torch.int32)
             self.z_lut = lut.to(self._device)
-        self._species_cache = (None, None)
+        self._species_cache = (L.Seen(), None)
 
     def _species(self, atomic_numbers: torch.Tensor):
         if self.z_lut is None:
             return None
-        key = (atomic_numbers.data_ptr(), atomic_numbers._version, atomic_numbers.shape[0])
-        if self._species_cache[0] == key:
+        if self._species_cache[0].same(atomic_numbers):
             return self._species_cache[1]
         z = atomic_numbers.to(self.z_lut.device)
         if bool((z < 0).any() | (z >= len(self.z_lut)).any()):
@@ -99,7 +98,7 @@ class PairTableModel(ModelInterface):
         sp = self.z_lut[z].contiguous()
         if bool((sp < 0).any()):
             raise ValueError("atomic number not in the model's species table")
-        self._species_cache = (key, sp)
+        self._species_cache = (L.Seen(atomic_numbers), sp)
         return sp
 
     def forward(self, state, **_kwargs) -> dict[str, torch.Tensor]:

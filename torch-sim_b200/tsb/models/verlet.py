@@ -72,7 +72,7 @@ class VerletListModel(ModelInterface):
             self.prune = 0.0  # the whole list is within cutoff + skin anyway
         self.max_neighbors = int(max_neighbors)
         self.n_builds = 0
-        self._key = None
+        self._key = None          # what the batched lists are for
         self._last_single = False
         # graph-safe mode: the rebuild is decided on the device (no host reads),
         # list overflow is recorded in a sticky device flag (see set_graph_safe)
@@ -85,12 +85,9 @@ class VerletListModel(ModelInterface):
     def _ensure(self, state, pos, cell_row):
         n, ns = state.n_atoms, state.n_systems
         sysi, z = state.system_idx, state.atomic_numbers
-        # the species and the table's cutoffs decide which pairs are listed; the tensors
-        # are held below, so that no other one can come to lie at the same address
-        table = self.model.table
-        key = (n, ns, pos.dtype, pos.device, sysi.data_ptr(), sysi._version, z.data_ptr(),
-               z._version, table.data_ptr(), table._version)
-        if self._key == key:
+        # the systems, the species and the table's cutoffs decide which pairs are listed
+        key, of = (n, ns, pos.dtype, pos.device), (sysi, z, self.model.table)
+        if (self._key == key and all(a.same(b) for a, b in zip(self._seen, of, strict=True))):
             return
         dev = pos.device
         rcs = self.model.cutoff + self.skin
@@ -109,7 +106,7 @@ class VerletListModel(ModelInterface):
                               device=dev)
         self._reset(n, ns, dev)
         self._built = False
-        self._key, self._listed = key, (sysi, z, table)
+        self._key, self._seen = key, tuple(map(L.Seen, of))
 
     def _reset(self, n, ns, dev):
         L.call("tsb_vlist_reset", n, ns, L.ptr(self.ws), self.ws.numel(), L.stream_ptr(dev))
