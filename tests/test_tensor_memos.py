@@ -97,3 +97,14 @@ def test_what_counts_as_the_same_tensor():
     assert not copy.deepcopy(seen).same(a) and not pickle.loads(pickle.dumps(seen)).same(a)
     a[0] = 5
     assert not seen.same(a) and not L.Seen().same(a)
+
+
+def test_what_counts_as_the_same_periodic_axes():
+    for flags in (True, [True] * 3, torch.tensor([True] * 3), torch.tensor(True)):
+        seen = L.SeenPbc(flags)
+        assert seen.same(flags) and not seen.same([True, False, True]) and not seen.same(False)
+    assert L.SeenPbc([True, False, True]).same(torch.tensor([1, 0, 1]))
+    cpu = torch.tensor([True] * 3)
+    seen = L.SeenPbc(cpu)
+    cpu[1] = False
+    assert not seen.same(cpu) and not L.SeenPbc().same(cpu)

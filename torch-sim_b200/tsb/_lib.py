@@ -271,9 +271,9 @@ def pbc_rows(pbc, n_systems: int, device) -> torch.Tensor:
     Flags given on the host (a bool, a list or a CPU tensor) are converted once
     and cached per (flags, S, device), so later calls -- inside a CUDA-graph
     capture too -- copy nothing from the host."""
-    if not (torch.is_tensor(pbc) and pbc.device.type == "cuda"):
-        flags = torch.as_tensor(pbc).reshape(-1).tolist()
-        key = (tuple(bool(f) for f in flags), int(n_systems), str(torch.device(device)))
+    flags = host_pbc(pbc)
+    if flags is not None:
+        key = (flags, int(n_systems), str(torch.device(device)))
         hit = _PBC_CACHE.get(key)
         if hit is None:
             if len(_PBC_CACHE) > 64:
@@ -282,6 +282,43 @@ def pbc_rows(pbc, n_systems: int, device) -> torch.Tensor:
             _PBC_CACHE[key] = hit
         return hit
     return _pbc_rows(pbc, n_systems)
+
+
+def host_pbc(pbc):
+    """The flags as a tuple when they are given on the host, None for a device tensor."""
+    if torch.is_tensor(pbc) and pbc.device.type == "cuda":
+        return None
+    return tuple(bool(f) for f in torch.as_tensor(pbc).reshape(-1).tolist())
+
+
+class SeenPbc:
+    """Periodic flags that something was worked out for: host flags by their values, a
+    device tensor as ``Seen``, and by its values (a device read) when another one comes."""
+
+    def __init__(self, pbc=None):
+        self.flags = None if pbc is None else host_pbc(pbc)
+        self.tensor = Seen() if pbc is None or self.flags is not None else Seen(pbc)
+        self.values = self.tensor.t.clone() if self.tensor.t is not None else None
+
+    def __reduce__(self):
+        return SeenPbc, ()
+
+    def __deepcopy__(self, _memo):
+        return SeenPbc()
+
+    def same(self, pbc) -> bool:
+        flags = host_pbc(pbc)
+        if flags is not None:
+            return flags == self.flags
+        if self.values is None:
+            return False
+        if self.tensor.same(pbc):
+            return True
+        v = self.values
+        if (pbc.device, pbc.dtype) != (v.device, v.dtype) or not torch.equal(pbc, v):
+            return False
+        self.tensor = Seen(pbc)
+        return True
 
 
 def _pbc_rows(p: torch.Tensor, n_systems: int) -> torch.Tensor:

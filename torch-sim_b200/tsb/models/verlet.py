@@ -73,6 +73,7 @@ class VerletListModel(ModelInterface):
         self.max_neighbors = int(max_neighbors)
         self.n_builds = 0
         self._key = None          # what the batched lists are for
+        self._pbc_of_single = L.SeenPbc()  # the flags that _pbc_all says it for
         self._last_single = False
         # graph-safe mode: the rebuild is decided on the device (no host reads),
         # list overflow is recorded in a sticky device flag (see set_graph_safe)
@@ -85,9 +86,11 @@ class VerletListModel(ModelInterface):
     def _ensure(self, state, pos, cell_row):
         n, ns = state.n_atoms, state.n_systems
         sysi, z = state.system_idx, state.atomic_numbers
-        # the systems, the species and the table's cutoffs decide which pairs are listed
+        # the systems, the species, the table's cutoffs and the periodic axes decide which
+        # pairs are listed
         key, of = (n, ns, pos.dtype, pos.device), (sysi, z, self.model.table)
-        if (self._key == key and all(a.same(b) for a, b in zip(self._seen, of, strict=True))):
+        if (self._key == key and all(a.same(b) for a, b in zip(self._seen, of, strict=True))
+                and self._seen_pbc.same(state.pbc)):
             return
         dev = pos.device
         rcs = self.model.cutoff + self.skin
@@ -107,6 +110,7 @@ class VerletListModel(ModelInterface):
         self._reset(n, ns, dev)
         self._built = False
         self._key, self._seen = key, tuple(map(L.Seen, of))
+        self._seen_pbc = L.SeenPbc(state.pbc)
 
     def _reset(self, n, ns, dev):
         L.call("tsb_vlist_reset", n, ns, L.ptr(self.ws), self.ws.numel(), L.stream_ptr(dev))
@@ -261,9 +265,8 @@ class VerletListModel(ModelInterface):
                 or self.per_atom_stresses):
             return False
         pbc = state.pbc
-        key = (pbc.data_ptr(), pbc._version) if isinstance(pbc, torch.Tensor) else bool(pbc)
-        if getattr(self, "_pbc_key", None) != key:  # one device read per pbc tensor
-            self._pbc_key = key
+        if not self._pbc_of_single.same(pbc):  # one device read per pbc tensor
+            self._pbc_of_single = L.SeenPbc(pbc)
             self._pbc_all = bool(L.pbc_rows(pbc, 1, state.positions.device).all())
         return self._pbc_all
 
