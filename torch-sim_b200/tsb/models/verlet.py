@@ -80,7 +80,7 @@ class VerletListModel(ModelInterface):
         self.graph_safe = False
         self.sticky = None
         self._built = False       # the batched lists have been built once
-        self._flags_host = None   # pinned copy of the flags, and when it is complete
+        self._flags_host = None   # pinned copy of the flags
 
     # -------------------------------------------------------------- buffers
     def _ensure(self, state, pos, cell_row):
@@ -156,19 +156,26 @@ class VerletListModel(ModelInterface):
         self._publish(flags).synchronize()
         return self._flags_host.tolist()
 
-    def _send_flags(self, flags) -> None:
-        self._flags_sent = torch.cuda.Event()
-        self._flags_sent.record(self._publish(flags))
+    def _send_flags(self, flags) -> torch.cuda.Event:
+        """The flags on their way: an event for _read_flags."""
+        sent = torch.cuda.Event()
+        sent.record(self._publish(flags))
+        return sent
 
-    def _read_flags(self) -> list[int]:
-        self._flags_sent.synchronize()
+    def _read_flags(self, sent) -> list[int]:
+        sent.synchronize()
         return self._flags_host.tolist()
+
+    def __getstate__(self):
+        # a copied or loaded model pins a buffer of its own (a copy of this one would be
+        # pageable memory, which the kernel must not write to)
+        return self.__dict__ | {"_flags_host": None}
 
     # ---------------------------------------------------------------- lists
     def _update_lists(self, state, pos, cell_row, pbc, sysi, species, active,
-                      table) -> bool:
-        """True when the flags are on their way and have to be read after the forces
-        have been launched."""
+                      table):
+        """None, or the event of flags on their way, which have to be read after the
+        forces have been launched."""
         n, ns, dev = state.n_atoms, state.n_systems, pos.device
         m, cutoff = self.model, self.model.cutoff
 
@@ -184,14 +191,13 @@ class VerletListModel(ModelInterface):
                                        self.prune, self.flags, self.ws)
             build()
             torch.maximum(self.sticky, self.flags[1:], out=self.sticky)
-            return False
+            return None
         if self._built and n >= self.UNREAD_ATOMS:
             # (the rebuild touches only the systems that the check marked)
             torch.ops.tsb.vlist_check_(pos, cell_row, sysi, active, ns, cutoff, self.skin,
                                        self.prune, self.flags, self.ws)
             build()
-            self._send_flags(self.flags)
-            return True
+            return self._send_flags(self.flags)
         while True:
             torch.ops.tsb.vlist_check_(pos, cell_row, sysi, active, ns, cutoff, self.skin,
                                        self.prune, self.flags, self.ws)
@@ -204,7 +210,7 @@ class VerletListModel(ModelInterface):
                 break
             self._grow_lists(st, n, ns, dev)
         self._built = True
-        return False
+        return None
 
     def _grow_lists(self, needed, n, ns, dev):
         """A list overflowed: regrow it and mark every system for a rebuild."""
@@ -252,7 +258,7 @@ class VerletListModel(ModelInterface):
         try:
             evaluate()
         finally:  # (the host buffer is in use until it has been read)
-            marked, overflow = self._read_flags() if pending else (0, 0)
+            marked, overflow = self._read_flags(pending) if pending else (0, 0)
         self.n_builds += 1 if marked else 0
         if overflow:
             self._grow_lists(overflow, state.n_atoms, n_sys, pos.device)
@@ -335,8 +341,7 @@ class VerletListModel(ModelInterface):
         if fresh:
             self._s_build(state, pos)
         self._s_check(state, pos, cell64)
-        if not fresh:
-            self._send_flags(self.s_expired)
+        sent = None if fresh else self._send_flags(self.s_expired)
         dt = pos.dtype
         energy = torch.empty(1, dtype=dt, device=state.device) if energy is None else energy
         forces = torch.empty_like(pos) if forces is None else forces
@@ -357,7 +362,7 @@ class VerletListModel(ModelInterface):
         try:
             evaluate()
         finally:  # (the host buffer is in use until it has been read)
-            expired = not fresh and self._read_flags()[0]
+            expired = sent is not None and self._read_flags(sent)[0]
         if expired:
             self._s_build(state, pos)
             self._s_check(state, pos, cell64)
