@@ -36,12 +36,19 @@ from .pair_potential import PairTableModel
 
 class VerletListModel(ModelInterface):
     # Batches of this many atoms have their lists rebuilt (the marked systems') without
-    # waiting for the check, smaller ones after reading its answer.  A FIRE step of Kob-
-    # Andersen systems, unread against read: 229 and 200 us at 6,000 atoms (the launches of
-    # a build that does nothing, with the host as the bound), 239 and 222 at 177,000, 290
-    # and 290 at 312,000, 343 and 363 at 422,000, 403 and 432 at 550,000 (the wait leaves
-    # the GPU idle).
+    # waiting for the check, smaller ones after reading its answer: below it the launches
+    # of a build that does nothing cost more than the wait, which leaves the GPU idle.  A
+    # FIRE step of Kob-Andersen systems of 64 to 1000 atoms, unread against read: 229 and
+    # 200 us at 6,000 atoms, 239 and 222 at 177,000, 290 and 290 at 312,000, 403 and 432 at
+    # 550,000 on one host; 239 and 253 at 211,000, 283 and 286 at 266,000, 294 and 314 at
+    # 330,000, 399 and 427 at 550,000 on another (FP64: 312 and 327, 378 and 399, 436 and
+    # 457, 637 and 666).
+    # Only with systems of at most UNREAD_SYSTEM_ATOMS, which are binned one block each, the
+    # marked ones alone (tsb_vlist_build): a larger one bins the whole batch in every call.
+    # NVE steps, unread against read: one system of 500,000 atoms in FP64 533 and 468 us,
+    # two of 200,000 335 and 275; 100 of 4,000 259 to 306 and 342 to 373.
     UNREAD_ATOMS = 262144
+    UNREAD_SYSTEM_ATOMS = 4096
 
     def __init__(self, model: PairTableModel, *, skin: float = 1.0, max_neighbors: int = 0,
                  prune: float | None = None):
@@ -192,7 +199,8 @@ class VerletListModel(ModelInterface):
             build()
             torch.maximum(self.sticky, self.flags[1:], out=self.sticky)
             return None
-        if self._built and n >= self.UNREAD_ATOMS:
+        if (self._built and n >= self.UNREAD_ATOMS
+                and self.max_system_atoms <= self.UNREAD_SYSTEM_ATOMS):
             # (the rebuild touches only the systems that the check marked)
             torch.ops.tsb.vlist_check_(pos, cell_row, sysi, active, ns, cutoff, self.skin,
                                        self.prune, self.flags, self.ws)
