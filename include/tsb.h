@@ -185,6 +185,13 @@ int tsb_verlet_forces(int potential, const double *table, int n_species,
                       void *energy, void *forces, void *stress, double *e_atom,
                       double *vir_atom, void *workspace, size_t workspace_bytes,
                       void *stream);
+/* The same, for a caller that launches it before it knows whether the list is good:
+ * nothing is written when *skip (the `expired` of the check, say) is not zero. */
+int tsb_verlet_forces_unless(int potential, const double *table, int n_species,
+                             const uint32_t *list, const int32_t *counts, int64_t n_atoms,
+                             const double *cell_row, int dtype, double cutoff, int out_flags,
+                             void *energy, void *forces, void *stress, const int32_t *skip,
+                             void *workspace, size_t workspace_bytes, void *stream);
 
 /* ---- anisotropic NPT Langevin (per-axis strains) ---------------------------
  * npt_langevin_anisotropic_step (torch_sim/integrators/npt.py:513-650): strains
@@ -365,6 +372,16 @@ int tsb_vlist_forces(int potential, const double *table, int n_species, const in
                      double prune_skin, int out_flags, void *energy, void *forces, void *stress,
                      void *energies, void *stresses, void *workspace, size_t workspace_bytes,
                      void *stream);
+/* The same, for a caller that launches it before it has read the build's flags: nothing
+ * is written to the results when *skip (flags + 1, say) is not zero. */
+int tsb_vlist_forces_unless(int potential, const double *table, int n_species,
+                            const int32_t *species, uint32_t *list, const int32_t *counts,
+                            const void *positions, const void *cell_row,
+                            const int64_t *system_idx, const uint8_t *sys_active,
+                            int64_t n_atoms, int64_t n_systems, int dtype, double cutoff,
+                            double prune_skin, int out_flags, void *energy, void *forces,
+                            void *stress, void *energies, void *stresses, const int32_t *skip,
+                            void *workspace, size_t workspace_bytes, void *stream);
 
 /* ---- adjoint of NVE trajectories (species-matrix LJ, FP64) ---------------
  * No kernel of the reference corresponds: it differentiates trajectories with

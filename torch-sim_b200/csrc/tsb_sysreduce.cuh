@@ -26,10 +26,10 @@ __device__ inline void write_sys(const SysGeom &G, const double *t, int flags, i
 template <class P>
 __global__ void k_sys_reduce(const SysGeom *g, const double *e_half, const double *vir_half,
                              int flags, P *energy, P *stress, const uint8_t *sys_active,
-                             int chunks, double *part) {
+                             int chunks, double *part, const int32_t *skip = nullptr) {
   __shared__ double sh[7][kBlock / 32];
   const int s = blockIdx.x, ch = blockIdx.y;
-  if (sys_active && !sys_active[s]) return;
+  if ((sys_active && !sys_active[s]) || (skip && *skip)) return;
   const SysGeom &G = g[s];
   const int64_t step = (G.count + chunks - 1) / chunks;
   const int64_t lo = (int64_t)ch * step;
@@ -61,9 +61,10 @@ __global__ void k_sys_reduce(const SysGeom *g, const double *e_half, const doubl
 
 template <class P>
 __global__ void k_sys_final(const SysGeom *g, const double *part, int64_t ns, int chunks,
-                            int flags, P *energy, P *stress, const uint8_t *sys_active) {
+                            int flags, P *energy, P *stress, const uint8_t *sys_active,
+                            const int32_t *skip = nullptr) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns || (sys_active && !sys_active[s])) return;
+  if (s >= ns || (sys_active && !sys_active[s]) || (skip && *skip)) return;
   double t[7] = {0, 0, 0, 0, 0, 0, 0};
   for (int c = 0; c < chunks; ++c)
     for (int k = 0; k < 7; ++k) t[k] += part[7 * (s * chunks + c) + k];

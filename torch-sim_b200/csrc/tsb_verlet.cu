@@ -261,7 +261,8 @@ __global__ void __launch_bounds__(256, 3)
                     const int32_t *__restrict__ raw, const uint32_t *__restrict__ list,
                     const int32_t *__restrict__ cnt, int64_t n, const double *__restrict__ cell,
                     const double *__restrict__ table, int ns_species, double cutoff,
-                    int flags, P *forces, double *part) {
+                    int flags, P *forces, double *part, const int32_t *skip) {
+  if (skip && *skip) return;  // (the list is no good: nothing is written)
   // (16-byte aligned rows and shifts are read in 16-byte pieces)
   __shared__ alignas(16) PairPrm<float> prm[kMaxSpecies * kMaxSpecies];
   __shared__ double prc2[kMaxSpecies * kMaxSpecies];
@@ -311,7 +312,8 @@ constexpr int kVerletFinal = 7 * 4 * 32;
 template <class P>
 __global__ void __launch_bounds__(kVerletFinal)
     k_verlet_final(const double *part, int64_t n_blocks, int flags, const double *cell,
-                   P *energy, P *stress) {
+                   P *energy, P *stress, const int32_t *skip) {
+  if (skip && *skip) return;
   __shared__ double sh[7][4];
   const int warp = threadIdx.x >> 5, k = warp >> 2, quarter = warp & 3;
   const int64_t step = (n_blocks + 3) / 4, lo = quarter * step;
@@ -434,17 +436,18 @@ extern "C" int tsb_verlet_check(const void *positions, const double *ref_positio
   return TSB_OK;
 }
 
-extern "C" int tsb_verlet_forces(int potential, const double *table, int n_species,
-                                 const uint32_t *list, const int32_t *counts, int64_t n_atoms,
-                                 const double *cell_row, int dtype, double cutoff,
-                                 int out_flags, void *energy, void *forces, void *stress,
-                                 double *e_atom, double *vir_atom, void *workspace,
-                                 size_t workspace_bytes, void *stream) {
+extern "C" int tsb_verlet_forces_unless(int potential, const double *table, int n_species,
+                                        const uint32_t *list, const int32_t *counts,
+                                        int64_t n_atoms, const double *cell_row, int dtype,
+                                        double cutoff, int out_flags, void *energy,
+                                        void *forces, void *stress, const int32_t *skip,
+                                        void *workspace, size_t workspace_bytes,
+                                        void *stream) {
   if (potential < TSB_POT_LJ || potential > TSB_POT_SOFT || n_species < 1 ||
       n_species > kMaxSpecies || !table || n_atoms < 1 || !list || !counts || !cell_row ||
-      !energy || !forces || !e_atom)
+      !energy || !forces)
     return TSB_ERR_INVALID_ARG;
-  if ((out_flags & TSB_OUT_STRESS) && (!stress || !vir_atom)) return TSB_ERR_INVALID_ARG;
+  if ((out_flags & TSB_OUT_STRESS) && !stress) return TSB_ERR_INVALID_ARG;
   Carver c(workspace, workspace_bytes);
   VerletWork w;
   carve_verlet(c, w, n_atoms);
@@ -453,10 +456,10 @@ extern "C" int tsb_verlet_forces(int potential, const double *table, int n_speci
 #define TSB_VF(POT, P)                                                                      \
   k_verlet_forces<POT, P><<<grid_for(n_atoms, kVerletBlock), kVerletBlock, 0, st>>>(      \
       w.wpos, w.pos4, w.raw, list, counts, n_atoms, cell_row, table, n_species, cutoff,   \
-      out_flags, (P *)forces, w.part);                                                     \
+      out_flags, (P *)forces, w.part, skip);                                               \
   k_verlet_final<P><<<1, kVerletFinal, 0, st>>>(w.part, grid_for(n_atoms, kVerletBlock),   \
                                                 out_flags, cell_row, (P *)energy,          \
-                                                (P *)stress);
+                                                (P *)stress, skip);
   if (dtype == TSB_F64) {
     if (potential == TSB_POT_LJ) { TSB_VF(TSB_POT_LJ, double) }
     else if (potential == TSB_POT_MORSE) { TSB_VF(TSB_POT_MORSE, double) }
@@ -471,6 +474,18 @@ extern "C" int tsb_verlet_forces(int potential, const double *table, int n_speci
 #undef TSB_VF
   TSB_CHECK_LAUNCH();
   return TSB_OK;
+}
+
+extern "C" int tsb_verlet_forces(int potential, const double *table, int n_species,
+                                 const uint32_t *list, const int32_t *counts, int64_t n_atoms,
+                                 const double *cell_row, int dtype, double cutoff,
+                                 int out_flags, void *energy, void *forces, void *stress,
+                                 double *e_atom, double *vir_atom, void *workspace,
+                                 size_t workspace_bytes, void *stream) {
+  if (!e_atom || ((out_flags & TSB_OUT_STRESS) && !vir_atom)) return TSB_ERR_INVALID_ARG;
+  return tsb_verlet_forces_unless(potential, table, n_species, list, counts, n_atoms, cell_row,
+                                  dtype, cutoff, out_flags, energy, forces, stress, nullptr,
+                                  workspace, workspace_bytes, stream);
 }
 
 namespace tsb {

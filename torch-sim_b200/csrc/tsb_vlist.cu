@@ -603,7 +603,8 @@ __global__ void __launch_bounds__(kVlBlock)
                 const float *__restrict__ band, const double *__restrict__ table,
                 int ns_species, double cutoff, int flags, P *forces, P *energies, P *stresses,
                 const SysGeom *__restrict__ cur, double *e_half, double *vir_half,
-                const uint8_t *__restrict__ active) {
+                const uint8_t *__restrict__ active, const int32_t *skip) {
+  if (skip && *skip) return;  // (the lists are no good: nothing is written)
   constexpr bool F32 = sizeof(R) == 4;
   using Pos4 = std::conditional_t<F32, float4, double4>;
   using Sh = std::conditional_t<F32, float4, double>;  // per shift: one, or three
@@ -890,16 +891,18 @@ template <int POT, class R, class P>
 static void vl_launch(VlWork &w, const uint32_t *list, const int32_t *counts, int64_t n,
                       const int64_t *sys, const double *table, int nsp, double cutoff,
                       int flags, P *forces, P *energies, P *stresses, const uint8_t *active,
-                      cudaStream_t st) {
+                      const int32_t *skip, cudaStream_t st) {
   if (n <= kGroupSearchMaxAtoms)
     k_vl_forces<POT, R, P, kSearchGroup><<<grid_for(kSearchGroup * n, kVlBlock), kVlBlock, 0,
                                             st>>>(
         w.wpos, w.wpos32, list, counts, n, w.perm, sys, w.sv, w.svf, w.band, table, nsp,
-        cutoff, flags, forces, energies, stresses, w.cur, w.e_half, w.vir_half, active);
+        cutoff, flags, forces, energies, stresses, w.cur, w.e_half, w.vir_half, active,
+        skip);
   else
     k_vl_forces<POT, R, P, 1><<<grid_for(n, kVlBlock), kVlBlock, 0, st>>>(
         w.wpos, w.wpos32, list, counts, n, w.perm, sys, w.sv, w.svf, w.band, table, nsp,
-        cutoff, flags, forces, energies, stresses, w.cur, w.e_half, w.vir_half, active);
+        cutoff, flags, forces, energies, stresses, w.cur, w.e_half, w.vir_half, active,
+        skip);
 }
 
 template <class P>
@@ -907,7 +910,8 @@ static int vl_forces(int pot, const double *table, int nsp, const int32_t *speci
                      uint32_t *list, const int32_t *counts, const P *pos, const P *cell,
                      const int64_t *sys, const uint8_t *active, int64_t n, int64_t ns,
                      double cutoff, double prune, int flags, P *energy, P *forces, P *stress,
-                     P *energies, P *stresses, VlWork &w, cudaStream_t st) {
+                     P *energies, P *stresses, const int32_t *skip, VlWork &w,
+                     cudaStream_t st) {
   vl_geom_frame<P>(pos, cell, sys, species, nsp, n, ns, cutoff, w, st);
   if (prune > 0.0) {
     // systems marked by the check or rebuilt since their last pruning form their
@@ -923,10 +927,10 @@ static int vl_forces(int pot, const double *table, int nsp, const int32_t *speci
 #define TSB_VLL(POT)                                                                        \
   if (f64)                                                                                  \
     vl_launch<POT, double, P>(w, list, counts, n, sys, table, nsp, cutoff, flags, forces,  \
-                              energies, stresses, active, st);                              \
+                              energies, stresses, active, skip, st);                        \
   else                                                                                      \
     vl_launch<POT, float, P>(w, list, counts, n, sys, table, nsp, cutoff, flags, forces,   \
-                             energies, stresses, active, st);
+                             energies, stresses, active, skip, st);
   if (pot == TSB_POT_LJ) {
     TSB_VLL(TSB_POT_LJ)
   } else if (pot == TSB_POT_MORSE) {
@@ -936,10 +940,10 @@ static int vl_forces(int pot, const double *table, int nsp, const int32_t *speci
   }
 #undef TSB_VLL
   k_sys_reduce<P><<<dim3((unsigned)ns, (unsigned)w.chunks), kBlock, 0, st>>>(
-      w.cur, w.e_half, w.vir_half, flags, energy, stress, active, w.chunks, w.part);
+      w.cur, w.e_half, w.vir_half, flags, energy, stress, active, w.chunks, w.part, skip);
   if (w.chunks > 1)
     k_sys_final<P><<<grid_for(ns), kBlock, 0, st>>>(w.cur, w.part, ns, w.chunks, flags, energy,
-                                                     stress, active);
+                                                     stress, active, skip);
   TSB_CHECK_LAUNCH();
   return TSB_OK;
 }
@@ -1169,15 +1173,16 @@ extern "C" int tsb_vlist_build(const void *positions, const void *cell_row, cons
                                workspace_bytes, stream);
 }
 
-extern "C" int tsb_vlist_forces(int potential, const double *table, int n_species,
-                                const int32_t *species, uint32_t *list,
-                                const int32_t *counts, const void *positions,
-                                const void *cell_row, const int64_t *system_idx,
-                                const uint8_t *sys_active, int64_t n_atoms, int64_t n_systems,
-                                int dtype, double cutoff, double prune_skin, int out_flags,
-                                void *energy,
-                                void *forces, void *stress, void *energies, void *stresses,
-                                void *workspace, size_t workspace_bytes, void *stream) {
+extern "C" int tsb_vlist_forces_unless(int potential, const double *table, int n_species,
+                                       const int32_t *species, uint32_t *list,
+                                       const int32_t *counts, const void *positions,
+                                       const void *cell_row, const int64_t *system_idx,
+                                       const uint8_t *sys_active, int64_t n_atoms,
+                                       int64_t n_systems, int dtype, double cutoff,
+                                       double prune_skin, int out_flags, void *energy,
+                                       void *forces, void *stress, void *energies,
+                                       void *stresses, const int32_t *skip, void *workspace,
+                                       size_t workspace_bytes, void *stream) {
   if (potential < TSB_POT_LJ || potential > TSB_POT_SOFT || n_species < 1 ||
       n_species > kMaxSpecies || !table || n_atoms < 1 || n_systems < 1 || !list || !counts ||
       !positions || !cell_row || !system_idx || !energy || !(prune_skin >= 0.0))
@@ -1197,13 +1202,28 @@ extern "C" int tsb_vlist_forces(int potential, const double *table, int n_specie
                              (const double *)positions, (const double *)cell_row, system_idx,
                              sys_active, n_atoms, n_systems, cutoff, prune_skin, out_flags,
                              (double *)energy, (double *)forces, (double *)stress,
-                             (double *)energies, (double *)stresses, w, st);
+                             (double *)energies, (double *)stresses, skip, w, st);
   if (dtype == TSB_F32)
     return vl_forces<float>(potential, table, n_species, species, list, counts,
                             (const float *)positions, (const float *)cell_row, system_idx,
                             sys_active, n_atoms, n_systems, cutoff, prune_skin, out_flags,
                             (float *)energy,
                             (float *)forces, (float *)stress, (float *)energies,
-                            (float *)stresses, w, st);
+                            (float *)stresses, skip, w, st);
   return TSB_ERR_INVALID_ARG;
+}
+
+extern "C" int tsb_vlist_forces(int potential, const double *table, int n_species,
+                                const int32_t *species, uint32_t *list,
+                                const int32_t *counts, const void *positions,
+                                const void *cell_row, const int64_t *system_idx,
+                                const uint8_t *sys_active, int64_t n_atoms, int64_t n_systems,
+                                int dtype, double cutoff, double prune_skin, int out_flags,
+                                void *energy, void *forces, void *stress, void *energies,
+                                void *stresses, void *workspace, size_t workspace_bytes,
+                                void *stream) {
+  return tsb_vlist_forces_unless(potential, table, n_species, species, list, counts, positions,
+                                 cell_row, system_idx, sys_active, n_atoms, n_systems, dtype,
+                                 cutoff, prune_skin, out_flags, energy, forces, stress, energies,
+                                 stresses, nullptr, workspace, workspace_bytes, stream);
 }

@@ -80,6 +80,8 @@ PROTOTYPES = {
                                 _vp]),
     "tsb_verlet_forces": (_int, [_int, _vp, _int, _vp, _vp, _i64, _vp, _int, _dbl, _int, _vp,
                                  _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
+    "tsb_verlet_forces_unless": (_int, [_int, _vp, _int, _vp, _vp, _i64, _vp, _int, _dbl, _int,
+                                        _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "tsb_npt_crescale_iso": (_int, [_vp, _vp, _vp, _vp, _i64, _i64, _int, _vp, _vp, _vp, _vp,
                                     _vp, _vp, _vp, _vp, _u64, _u64, _vp, _sz, _vp]),
     "tsb_npt_crescale_aniso": (_int, [_vp, _vp, _vp, _vp, _i64, _i64, _int, _vp, _vp, _vp,
@@ -111,6 +113,9 @@ PROTOTYPES = {
                                 _dbl, _vp, _vp, _vp, _sz, _vp, _sz, _vp]),
     "tsb_vlist_forces": (_int, [_int, _vp, _int, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64,
                                 _int, _dbl, _dbl, _int, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
+    "tsb_vlist_forces_unless": (_int, [_int, _vp, _int, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64,
+                                       _i64, _int, _dbl, _dbl, _int, _vp, _vp, _vp, _vp, _vp,
+                                       _vp, _vp, _sz, _vp]),
     "tsb_fire_workspace_size": (_sz, [_i64]),
     "tsb_fire_ase_pre": (_int, _FIRE_ARGS),
     "tsb_fire_vv_pre": (_int, _FIRE_ARGS),

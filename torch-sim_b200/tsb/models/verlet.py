@@ -13,9 +13,9 @@ small ones whose atoms and cells move (FIRE with a cell filter, NPT, MD).
 Every periodic cell must be at least cutoff + skin wide (image shifts in
 {-1,0,1}^3); narrower cells raise ValueError.  The wrapper keeps its own device
 workspace (the list frame) and reads two flags from the device per call, while the
-force kernel runs: the flags leave for pinned memory before it is launched, and a call
-whose lists turn out to have overflowed (or, for one large system, expired) is
-evaluated again before it returns.
+force kernel runs: the flags leave for pinned memory before it is launched.  Where the
+lists turn out to have overflowed (or, for one large system, expired) that kernel has
+written nothing, and the call evaluates again before it returns or raises.
 
 One fully periodic system with FP32 pair arithmetic and no per-atom outputs (the
 500,000-atom workload) takes the single-system kernels (tsb_verlet_build /
@@ -223,6 +223,7 @@ class VerletListModel(ModelInterface):
     def _grow_lists(self, needed, n, ns, dev):
         """A list overflowed: regrow it and mark every system for a rebuild."""
         if needed >= (1 << 30):
+            self._key = None  # (what has been listed is no good for a later call either)
             raise ValueError("VerletListModel needs every periodic cell width >= "
                              "cutoff + skin")
         self.cap = int(needed * 1.2) + 8
@@ -257,14 +258,14 @@ class VerletListModel(ModelInterface):
         if m.precision == "fp64":
             flags |= L.MATH_FP64
 
-        def evaluate():
+        def evaluate(skip=None):
             torch.ops.tsb.vlist_forces_(m.kind, table, m.n_species, species, self.list,
                                         self.counts, pos, cell_row, sysi, active, n_sys,
                                         m.cutoff, self.prune, flags, energy, forces, stress,
-                                        energies, stresses, self.ws)
+                                        energies, stresses, self.ws, skip)
 
         try:
-            evaluate()
+            evaluate(self.flags[1:] if pending else None)
         finally:  # (the host buffer is in use until it has been read)
             marked, overflow = self._read_flags(pending) if pending else (0, 0)
         self.n_builds += 1 if marked else 0
@@ -315,6 +316,7 @@ class VerletListModel(ModelInterface):
 
     def _s_build(self, state, pos):
         cell = state.cell[0].mT.to(pos.dtype).contiguous()
+        self._s_built = False
         while True:
             L.call("tsb_verlet_build", L.ptr(pos), L.ptr(cell), state.n_atoms,
                    L.dtype_code(pos.dtype), self.model.cutoff, self.skin, L.ptr(self.s_list),
@@ -360,15 +362,15 @@ class VerletListModel(ModelInterface):
         flags = L.OUT_FORCES | (L.OUT_STRESS if stress is not None else 0)
         m = self.model
 
-        def evaluate():
-            L.call("tsb_verlet_forces", m.kind, L.ptr(m.table), m.n_species,
+        def evaluate(skip=None):
+            L.call("tsb_verlet_forces_unless", m.kind, L.ptr(m.table), m.n_species,
                    L.ptr(self.s_list), L.ptr(self.s_counts), state.n_atoms, L.ptr(cell64),
                    L.dtype_code(dt), m.cutoff, flags, L.ptr(energy), L.ptr(forces),
-                   L.ptr(stress), L.ptr(self.s_e_atom), L.ptr(self.s_vir_atom),
-                   L.ptr(self.s_ws), self.s_ws.numel(), L.stream_ptr(state.device))
+                   L.ptr(stress), L.ptr(skip), L.ptr(self.s_ws), self.s_ws.numel(),
+                   L.stream_ptr(state.device))
 
         try:
-            evaluate()
+            evaluate(None if fresh else self.s_expired)
         finally:  # (the host buffer is in use until it has been read)
             expired = sent is not None and self._read_flags(sent)[0]
         if expired:

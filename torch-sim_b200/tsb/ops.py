@@ -318,21 +318,23 @@ _define("vlist_build_(Tensor positions, Tensor cell_row, Tensor pbc, Tensor syst
 
 def _vlist_forces(kind, table, n_species, species, lst, counts, positions, cell_row,
                   system_idx, sys_active, n_systems, cutoff, prune, flags, energy, forces,
-                  stress, energies, stresses, workspace):
+                  stress, energies, stresses, workspace, skip=None):
     nz = lambda t: _P(t) if (t is not None and t.numel()) else None  # noqa: E731
-    L.call("tsb_vlist_forces", int(kind), _P(table), int(n_species), _P(species), _P(lst),
+    L.call("tsb_vlist_forces_unless", int(kind), _P(table), int(n_species), _P(species), _P(lst),
            _P(counts), _P(positions), _P(cell_row), _P(system_idx), _P(sys_active),
            positions.shape[0], int(n_systems), L.dtype_code(positions.dtype), float(cutoff),
            float(prune), int(flags), _P(energy), nz(forces), nz(stress), nz(energies),
-           nz(stresses), _P(workspace), workspace.numel(), _stream(positions))
+           nz(stresses), _P(skip), _P(workspace), workspace.numel(), _stream(positions))
 
 
+# nothing is written when skip (int32, on the device) is given and not zero;
 # with prune > 0 the lists are reordered in place (front parts), so nlist is written
 _define("vlist_forces_(int kind, Tensor table, int n_species, Tensor? species, "
         "Tensor(g!) nlist, Tensor counts, Tensor positions, Tensor cell_row, "
         "Tensor system_idx, Tensor? sys_active, int n_systems, float cutoff, float prune, "
         "int flags, Tensor(a!) energy, Tensor(b!)? forces, Tensor(c!)? stress, "
-        "Tensor(d!)? energies, Tensor(e!)? stresses, Tensor(f!) workspace) -> ()",
+        "Tensor(d!)? energies, Tensor(e!)? stresses, Tensor(f!) workspace, "
+        "Tensor? skip=None) -> ()",
         _vlist_forces, _noop)
 
 
