@@ -167,7 +167,7 @@ int tsb_md_baoab_boa(void *positions, void *momenta, const void *forces,
  *   more than skin/2 or the cell differs from the build's (then rebuild and check
  *   again).  cell_row float64.
  * tsb_verlet_forces: energy [1], forces [N,3] (dtype), stress [1,3,3] with
- *   TSB_OUT_STRESS; e_atom [N] and vir_atom [N,6] are float64 scratch.  Uses the
+ *   TSB_OUT_STRESS.  e_atom and vir_atom are not used (NULL or anything).  Uses the
  *   workspace filled by tsb_verlet_check.  cell_row float64. */
 size_t tsb_verlet_workspace_size(int64_t n_atoms);
 int tsb_verlet_build(const void *positions, const void *cell_row, int64_t n_atoms, int dtype,

@@ -480,9 +480,8 @@ extern "C" int tsb_verlet_forces(int potential, const double *table, int n_speci
                                  const uint32_t *list, const int32_t *counts, int64_t n_atoms,
                                  const double *cell_row, int dtype, double cutoff,
                                  int out_flags, void *energy, void *forces, void *stress,
-                                 double *e_atom, double *vir_atom, void *workspace,
-                                 size_t workspace_bytes, void *stream) {
-  if (!e_atom || ((out_flags & TSB_OUT_STRESS) && !vir_atom)) return TSB_ERR_INVALID_ARG;
+                                 double * /*e_atom*/, double * /*vir_atom*/,
+                                 void *workspace, size_t workspace_bytes, void *stream) {
   return tsb_verlet_forces_unless(potential, table, n_species, list, counts, n_atoms, cell_row,
                                   dtype, cutoff, out_flags, energy, forces, stress, nullptr,
                                   workspace, workspace_bytes, stream);

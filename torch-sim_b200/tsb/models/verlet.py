@@ -301,8 +301,6 @@ class VerletListModel(ModelInterface):
         self.s_wraps = torch.empty((n, 3), dtype=torch.int32, device=dev)
         self.s_status = torch.zeros(1, dtype=torch.int32, device=dev)
         self.s_expired = torch.zeros(1, dtype=torch.int32, device=dev)
-        self.s_e_atom = torch.empty(n, dtype=torch.float64, device=dev)
-        self.s_vir_atom = torch.empty((n, 6), dtype=torch.float64, device=dev)
         self.s_ws = torch.empty(L.load().tsb_verlet_workspace_size(n), dtype=torch.uint8,
                                 device=dev)
         self._s_key = key
