@@ -417,11 +417,14 @@ int tsb_adj_kick(double *lam_p, const double *lam_q, const double *inv_m, double
  * recursion back over traj (lam_q, lam_p in place, grad_params [S, ns, ns, 2] +=;
  * `first`: traj starts at step 0, whose coefficient is dt / 2).  *status (int32, the
  * caller's, zero before) becomes the neighbour count that exceeded max_neighbors, or
- * 1 << 30 for a narrower cell or a system of more than max_system_atoms atoms; the
- * results of such systems are then meaningless.  max_system_atoms sizes the blocks: it
+ * 1 << 30 for a narrower cell or a system of more than max_system_atoms atoms (such a
+ * system's q_out and p_out are its q and p); the results are then meaningless.  max_system_atoms sizes the blocks: it
  * may be larger than the largest system, and a larger system is left out whole.  TSB_ERR_CAPACITY: the
  * lists do not fit a block's shared memory; TSB_ERR_UNSUPPORTED: too many atoms. */
 int tsb_adj_block_max_atoms(void);
+/* the longest lists (max_neighbors) whose block fits the current device's shared memory,
+ * for the sweep or the trajectory alone; 0: too many atoms or species */
+int tsb_adj_block_max_neighbors(int64_t max_system_atoms, int n_species, int sweep);
 size_t tsb_adj_block_workspace_size(int64_t n_systems);
 int tsb_adj_trajectory(const double *table, int n_species, const int32_t *species,
                        const double *cell_row, const uint8_t *pbc, const int64_t *system_idx,

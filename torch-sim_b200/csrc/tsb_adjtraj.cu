@@ -309,7 +309,15 @@ __global__ void __launch_bounds__(kBlkThreads, 2)
   BlkSmem S = blk_carve(smem, max_atoms, B.stride, B.cap, B.nsp, 0);
   BlkThread<LANES> t;
   blk_table(B, S);
-  if (!t.setup(B, S, blockIdx.x, max_atoms)) return;  // (the same for every thread)
+  if (!t.setup(B, S, blockIdx.x, max_atoms)) {  // (the same for every thread)
+    // the caller learns of it at the end: what it computes meanwhile reads real positions
+    const int64_t end = 3 * B.hi[blockIdx.x];
+    for (int64_t k = 3 * B.lo[blockIdx.x] + threadIdx.x; k < end; k += blockDim.x) {
+      q_out[k] = q0[k];
+      p_out[k] = p0[k];
+    }
+    return;
+  }
   const bool lead = t.on && t.lane == 0;
   double q[3], p[3], f[3], im = 0.0;
   for (int m = 0; m < 3; ++m) {
@@ -532,6 +540,17 @@ static void blk_room(K kernel, size_t bytes) {
 using namespace tsb;
 
 extern "C" int tsb_adj_block_max_atoms(void) { return kBlkMaxAtoms; }
+
+extern "C" int tsb_adj_block_max_neighbors(int64_t max_system_atoms, int n_species, int sweep) {
+  if (max_system_atoms < 1 || max_system_atoms > kBlkMaxAtoms || n_species < 1 ||
+      n_species > kBlkMaxSpecies)
+    return 0;
+  const int stride = (int)(max_system_atoms + 1) / 2 * 2;
+  const int64_t room = (int64_t)blk_smem_limit() -
+                       (int64_t)blk_bytes((int)max_system_atoms, stride, 0, n_species,
+                                          sweep ? 2 : 0);
+  return room > 0 ? (int)(room / (int64_t)(sizeof(uint16_t) * stride)) : 0;
+}
 
 extern "C" size_t tsb_adj_block_workspace_size(int64_t n_systems) {
   Carver c(nullptr, (size_t)-1);

@@ -61,6 +61,7 @@ PROTOTYPES = {
     "tsb_vv_kick": (_int, [_vp, _vp, _dbl, _vp, _i64, _vp]),
     "tsb_adj_kick": (_int, [_vp, _vp, _vp, _dbl, _i64, _vp]),
     "tsb_adj_block_max_atoms": (_int, []),
+    "tsb_adj_block_max_neighbors": (_int, [_i64, _int, _int]),
     "tsb_adj_block_workspace_size": (_sz, [_i64]),
     "tsb_adj_trajectory": (_int, [_vp, _int, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _dbl, _dbl,
                                   _int, _vp, _vp, _vp, _dbl, _i64, _i64, _vp, _vp, _vp, _vp,

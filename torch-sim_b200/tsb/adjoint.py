@@ -341,7 +341,8 @@ class _Blocks:
     ``tsb_adj_sweep``), for problems whose systems and lists fit a block: the list
     capacity, grown from the device's report, and the calls.  Raises _NoBlocks when
     they do not fit (too many atoms, a cell narrower than cutoff + skin, lists
-    beyond a block's shared memory); the caller then takes the graph path."""
+    beyond a block's shared memory); the caller then takes the graph path, and a later
+    call with the same problem takes it at once."""
 
     SKIN = 1.0
     CAP = 160            # neighbours per atom at first (argon at 9.5 A: ~100)
@@ -354,27 +355,34 @@ class _Blocks:
                 _Blocks.SKIN, cap, L.ptr(inv_m))
 
     @staticmethod
-    def run(P, body):
+    def capacity(P, sweep):
+        """List capacity to run with.  Raises _NoBlocks, before anything is allocated or
+        launched, for what is known not to fit: too many atoms or species, lists beyond a
+        block's shared memory (of the sweep too when there is one), and what an earlier
+        call of this problem has found (a narrow cell, or how long its lists are)."""
+        unfit = P.__dict__.get("_unfit")
+        cap = P.__dict__.get("_block_cap", _Blocks.CAP)
+        if (P.cell_row.dtype != torch.float64
+                or cap > L.load().tsb_adj_block_max_neighbors(P.max_sys, P.n_species, sweep)
+                or (unfit is not None and unfit[0] == P.cutoff and unfit[1].same(P.cell_row)
+                    and unfit[2].same(P.pbc))):
+            raise _NoBlocks
+        return cap
+
+    @staticmethod
+    def run(P, sweep, body):
         """``body(call)`` on this problem, again with longer lists
         while the device reports an overflow (one read at the end)."""
         lib, dev = L.load(), P.cell_row.device
-        if (P.max_sys > lib.tsb_adj_block_max_atoms() or P.n_species > 4
-                or P.cell_row.dtype != torch.float64):
-            raise _NoBlocks
+        cap = _Blocks.capacity(P, sweep)
         ws = L.Workspace.get(dev, lib.tsb_adj_block_workspace_size(P.n_systems))
         inv_m = (1.0 / P.masses).contiguous()
-        cap = P.__dict__.get("_block_cap", _Blocks.CAP)
         while True:
             status = torch.zeros(1, dtype=torch.int32, device=dev)
 
             def call(name, table, *args):
-                try:
-                    L.call(name, *_Blocks._common(P, table, cap, inv_m), *args, L.ptr(status),
-                           L.ptr(ws), ws.numel(), L.stream_ptr(dev))
-                except L.TsbError as e:
-                    if e.status == L.TSB_ERR_CAPACITY:
-                        raise _NoBlocks from None
-                    raise
+                L.call(name, *_Blocks._common(P, table, cap, inv_m), *args, L.ptr(status),
+                       L.ptr(ws), ws.numel(), L.stream_ptr(dev))
 
             out = body(call)
             needed = int(status.item())
@@ -382,8 +390,10 @@ class _Blocks:
                 P.__dict__["_block_cap"] = cap
                 return out
             if needed >= (1 << 30):
-                raise _NoBlocks
-            cap = needed + needed // 8 + 4
+                P.__dict__["_unfit"] = (P.cutoff, L.Seen(P.cell_row), L.Seen(P.pbc))
+            else:
+                P.__dict__["_block_cap"] = needed + needed // 8 + 4
+            cap = _Blocks.capacity(P, sweep)
 
     @staticmethod
     def _vec(t, P):
@@ -412,7 +422,7 @@ class _Blocks:
     @staticmethod
     def integrate(q0, p0, table, P, keep_checkpoints):
         q0, p0, table = _Blocks._vec(q0, P), _Blocks._vec(p0, P), table.contiguous()
-        return _Blocks.run(P, lambda call: _Blocks.trajectory(
+        return _Blocks.run(P, False, lambda call: _Blocks.trajectory(
             call, q0, p0, table, P, P.n_steps, ckpt=keep_checkpoints))
 
     @staticmethod
@@ -420,6 +430,7 @@ class _Blocks:
         """(loss, lam_q, lam_p, gpar).  While every step's positions fit TRAJ_BYTES
         they are kept and the sweep reads them; else each checkpoint segment is
         integrated again before its sweep (memory O(N T / k + N k))."""
+        _Blocks.capacity(P, True)
         q0, p0, table = _Blocks._vec(q0, P), _Blocks._vec(p0, P), table.contiguous()
         dev, f64, T = q0.device, torch.float64, P.n_steps
         whole = 8 * q0.numel() * T <= _Blocks.TRAJ_BYTES
@@ -442,7 +453,7 @@ class _Blocks:
                     _Blocks.sweep(call, seg, table, P, c == 0, lam_q, lam_p, gpar)
             return loss, lam_q, lam_p, gpar
 
-        return _Blocks.run(P, body)
+        return _Blocks.run(P, True, body)
 
 
 def _retry_on_overflow(fn, P, table):
