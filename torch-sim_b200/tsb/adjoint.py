@@ -12,8 +12,10 @@ histogram of the final frame; its backward runs the exact discrete adjoint:
                         lam_q += c_k J_F(q_k)^T lam_p,  g += c_k dF(q_k)/dtheta^T lam_p
     (c_k = dt, dt/2 at k = 0; J_F = -Hessian; the q_T term vanishes as lam_p = 0)
 
-re-integrating each 20-step segment from a stored checkpoint (positions and
-momenta every ``checkpoint_every`` steps), so memory is O(N * T / k + N * k).
+re-integrating each segment from a stored checkpoint (positions and momenta every
+``checkpoint_every`` = k steps, 20 by default), so memory is O(N * T / k + N * k).
+While the positions of every step take at most ``_Blocks.KEEP`` times what those
+checkpoints and one segment do, they are kept instead and nothing is integrated twice.
 The reference's own route (autograd through PairPotentialModel with
 retain_graph=True, pair_potential.py:420-425) omits J_F and gives wrong
 trajectory gradients; finite differences are the arbiter here.
@@ -346,7 +348,13 @@ class _Blocks:
 
     SKIN = 1.0
     CAP = 160            # neighbours per atom at first (argon at 9.5 A: ~100)
-    TRAJ_BYTES = 2 << 30  # positions of every step are kept up to this size
+    # The positions of every step are kept while they take at most KEEP times what the
+    # checkpoints and one segment would, and TRAJ_BYTES; else segments are integrated
+    # again.  256 systems of 108 atoms: 200 steps at the default of 20 per segment 7.3 ms
+    # and 129 MiB against 11.5 ms and 29 MiB; 1,000 steps (120 states against 1,000) 33 ms
+    # and 636 MiB against 54 ms and 80 MiB, so there the segments are taken.
+    KEEP = 8
+    TRAJ_BYTES = 2 << 30
 
     @staticmethod
     def _common(P, table, cap, inv_m):
@@ -426,16 +434,29 @@ class _Blocks:
             call, q0, p0, table, P, P.n_steps, ckpt=keep_checkpoints))
 
     @staticmethod
+    def keeps_all(n_steps, every, step_bytes):
+        """Are the positions of every step kept (``step_bytes`` each)?"""
+        kept = 2 * -(-n_steps // every) + min(every, n_steps)  # states of the other way
+        return (n_steps <= _Blocks.KEEP * kept
+                and n_steps * step_bytes <= _Blocks.TRAJ_BYTES)
+
+    @staticmethod
     def loss_and_grad(table, q0, p0, P):
-        """(loss, lam_q, lam_p, gpar).  While every step's positions fit TRAJ_BYTES
-        they are kept and the sweep reads them; else each checkpoint segment is
-        integrated again before its sweep (memory O(N T / k + N k))."""
+        """(loss, lam_q, lam_p, gpar).  While every step's positions are kept
+        (``keeps_all``) the sweep reads them; else, and where there is no room for them,
+        each checkpoint segment is integrated again before its sweep."""
         _Blocks.capacity(P, True)
         q0, p0, table = _Blocks._vec(q0, P), _Blocks._vec(p0, P), table.contiguous()
         dev, f64, T = q0.device, torch.float64, P.n_steps
-        whole = 8 * q0.numel() * T <= _Blocks.TRAJ_BYTES
-        length = T if whole else min(P.checkpoint_every, T)
-        traj = torch.empty((length, *q0.shape), dtype=f64, device=dev)
+        whole = _Blocks.keeps_all(T, P.checkpoint_every, 8 * q0.numel())
+        traj = None
+        if whole:
+            try:
+                traj = torch.empty((T, *q0.shape), dtype=f64, device=dev)
+            except torch.cuda.OutOfMemoryError:
+                whole = False
+        if traj is None:
+            traj = torch.empty((min(P.checkpoint_every, T), *q0.shape), dtype=f64, device=dev)
 
         def body(call):
             qT, _, ckpt = _Blocks.trajectory(call, q0, p0, table, P, T, ckpt=not whole,
