@@ -289,9 +289,9 @@ static void carve_pair(Carver &c, PairWork &w, int64_t n, int64_t ns) {
 constexpr int64_t kPairWarpMaxAtoms = 16384;
 
 template <int POT, class R, class P, bool VIR>
-static void launch_forces(PairWork &w, int64_t n, int64_t ns, const double *table, int nsp, double cutoff,
-                          int flags, P *forces, P *energies, P *stresses,
-                          const uint8_t *active, cudaStream_t st) {
+static int launch_forces(PairWork &w, int64_t n, int64_t ns, const double *table, int nsp,
+                         double cutoff, int flags, P *forces, P *energies, P *stresses,
+                         const uint8_t *active, cudaStream_t st) {
   using Warp = PairWarpSmem<R, P, VIR>;
   const size_t tab = (size_t)nsp * nsp * (sizeof(PairPrm<R>) + sizeof(double));
   auto room = [](auto kernel, size_t bytes) {
@@ -306,7 +306,7 @@ static void launch_forces(PairWork &w, int64_t n, int64_t ns, const double *tabl
         w.b, n, table, nsp, cutoff, flags, forces, energies, stresses, w.e_half, w.vir_half,
         active);
   } else {
-    window_tiles(w.b, n, ns, active, w.tl, st);
+    TSB_TRY(window_tiles(w.b, n, ns, active, w.tl, st));
     auto go = [&](auto kernel) {
       const size_t bytes = room(kernel, kWinWarps * sizeof(TileSmem<false>) + tab);
       kernel<<<tile_grid(kernel, bytes), 32 * kWinWarps, bytes, st>>>(
@@ -318,6 +318,8 @@ static void launch_forces(PairWork &w, int64_t n, int64_t ns, const double *tabl
     else
       go(k_pair_tile<POT, R, P, VIR, false>);
   }
+  TSB_CHECK_LAUNCH();
+  return TSB_OK;
 }
 
 template <class P>
@@ -333,26 +335,24 @@ static int pair_forward(int pot, const double *table, int nsp, const int32_t *sp
     const bool vir = flags & (TSB_OUT_STRESS | TSB_OUT_STRESSES);
     auto go = [&](auto pot_c) {
       constexpr int POT = decltype(pot_c)::value;
-      auto run = [&](auto kernel) {
-        kernel(w, n, ns, table, nsp, cutoff, flags, forces, energies, stresses, active, st);
+      auto run = [&](auto launch) {
+        return launch(w, n, ns, table, nsp, cutoff, flags, forces, energies, stresses, active,
+                      st);
       };
-      if (f64 && vir)
-        run(launch_forces<POT, double, P, true>);
-      else if (f64)
-        run(launch_forces<POT, double, P, false>);
-      else if (vir)
-        run(launch_forces<POT, float, P, true>);
-      else
-        run(launch_forces<POT, float, P, false>);
+      if (f64)
+        return vir ? run(launch_forces<POT, double, P, true>)
+                   : run(launch_forces<POT, double, P, false>);
+      return vir ? run(launch_forces<POT, float, P, true>)
+                 : run(launch_forces<POT, float, P, false>);
     };
     if (pot == TSB_POT_LJ)
-      go(std::integral_constant<int, TSB_POT_LJ>());
+      TSB_TRY(go(std::integral_constant<int, TSB_POT_LJ>()));
     else if (pot == TSB_POT_MORSE)
-      go(std::integral_constant<int, TSB_POT_MORSE>());
+      TSB_TRY(go(std::integral_constant<int, TSB_POT_MORSE>()));
     else if (pot == TSB_POT_SOFT)
-      go(std::integral_constant<int, TSB_POT_SOFT>());
+      TSB_TRY(go(std::integral_constant<int, TSB_POT_SOFT>()));
     else
-      go(std::integral_constant<int, TSB_POT_PLIFE>());
+      TSB_TRY(go(std::integral_constant<int, TSB_POT_PLIFE>()));
   }
   k_sys_reduce<P><<<dim3((unsigned)ns, (unsigned)w.chunks), kBlock, 0, st>>>(
       w.b.geom, w.e_half, w.vir_half, flags, energy, stress, active, w.chunks, w.part);
