@@ -552,7 +552,8 @@ constexpr int kTileColumns = 64;
 // first atom of its first non-empty row) makes the warp lay the column out: lane z
 // takes the bins at z of the column's rows.  Odd columns run backwards, so that the
 // order turns round at their ends.
-__global__ void k_window_tiles(BinData b, int64_t n, const uint8_t *sys_active, TileList t) {
+__global__ void k_window_tiles(BinData b, int64_t n, const uint8_t *sys_active, int width,
+                               TileList t) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -634,15 +635,15 @@ __global__ void k_window_tiles(BinData b, int64_t n, const uint8_t *sys_active, 
       done += __shfl_sync(full, inc, 31);
     }
     // tiles that start in the column
-    const int first = joined ? (at + 31) / 32 * 32 : at;
+    const int first = joined ? (at + width - 1) / width * width : at;
     const int end = at + total, limit = joined ? G.count : end;
-    const int nt = first < end ? (end - first + 31) / 32 : 0;
+    const int nt = first < end ? (end - first + width - 1) / width : 0;
     int k0 = 0;
     if (lane == 0 && nt > 0) k0 = atomicAdd(t.n_tiles, nt);
     k0 = __shfl_sync(full, k0, 0);
     for (int k = lane; k < nt; k += 32) {
-      const int o = first + 32 * k;
-      t.tiles[k0 + k] = Tile{base + o, min(32, limit - o), cs};
+      const int o = first + width * k;
+      t.tiles[k0 + k] = Tile{base + o, min(width, limit - o), cs};
     }
   }
 }
@@ -661,10 +662,10 @@ int restart_tiles(const TileList &t, cudaStream_t st) {
 }
 
 int window_tiles(const BinData &b, int64_t n, int64_t ns, const uint8_t *sys_active,
-                 const TileList &t, cudaStream_t st) {
+                 int width, const TileList &t, cudaStream_t st) {
   cudaMemsetAsync(t.n_tiles, 0, 2 * sizeof(int32_t), st);
   cudaMemsetAsync(t.cursor, 0, sizeof(int32_t) * ns, st);
-  k_window_tiles<<<grid_for(n), kBlock, 0, st>>>(b, n, sys_active, t);
+  k_window_tiles<<<grid_for(n), kBlock, 0, st>>>(b, n, sys_active, width, t);
   TSB_CHECK_LAUNCH();
   return TSB_OK;
 }

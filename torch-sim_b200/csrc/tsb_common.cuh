@@ -149,7 +149,7 @@ int prepare_bins_any(const P *positions, const P *cell_row, const uint8_t *pbc,
                      double search_cutoff, BinData &b, cudaStream_t st, const int32_t *species,
                      int64_t max_system_atoms);
 
-// Tiles of up to 32 neighbouring atoms for the tile-per-warp kernels
+// Tiles of up to `width` <= 32 neighbouring atoms for the tile-per-warp kernels
 // (tsb_window.cuh): tiles[0..*n_tiles) of the active systems, in any order (a tile's
 // results do not depend on it).
 struct Tile;
@@ -162,6 +162,6 @@ struct TileList {
 void carve_tiles(Carver &c, TileList &t, int64_t n_atoms, int64_t n_systems);
 int restart_tiles(const TileList &t, cudaStream_t st);  // before another pass over them
 int window_tiles(const BinData &b, int64_t n_atoms, int64_t n_systems, const uint8_t *sys_active,
-                 const TileList &t, cudaStream_t st);
+                 int width, const TileList &t, cudaStream_t st);
 
 }  // namespace tsb

@@ -3,8 +3,9 @@
 //
 // A warp works through the full neighbour set of an atom (candidates gathered by
 // tsb_window.cuh), so forces need no atomics and the summation order is fixed
-// (deterministic results).  Each unordered pair is evaluated from both ends; per-atom energies/virials take
-// half of each visit, matching the half-list weights of pair_potential.py:402-441.
+// (deterministic results).  Each unordered pair is evaluated from both ends; per-atom
+// energies/virials take half of each visit, matching the half-list weights of
+// pair_potential.py:402-441.
 // Displacements are formed in FP64 from the wrapped FP64 positions; the pair
 // function runs in R (float by default, double with TSB_MATH_FP64).
 #include "tsb_pair.cuh"
@@ -98,28 +99,48 @@ __device__ __forceinline__ void write_atom(int64_t i, const double *t, int flags
   }
 }
 
-template <class R, class P, bool VIR>
+// the pairs of one atom: displacement, species of the neighbour and, << 8, its offset in
+// its span modulo 4
+template <class R>
+struct PairWin : WinSpans {
+  static constexpr int kCap = 192;  // (more: several chunks)
+  R x[kCap], y[kCap], z[kCap];
+  uint16_t info[kCap];
+};
+
+template <class R, bool VIR>
 struct PairWarpSmem {
   // FP32 pair math: the force sums decide the result's digits, so their order is kept:
   // four partial sums per component, each over every fourth candidate of a span in turn,
   // as four lanes per atom would take them
   static constexpr bool ORDERED = sizeof(R) == 4;
   static constexpr int NA = VIR ? 10 : 4;  // forces, energy, virial
-  WinSmem win;
-  float4 term[ORDERED ? 32 : 1];
+  PairWin<R> win;
+  // the force terms of 32 pairs, each product rounded on its own (rows eleven banks
+  // apart, so that the lanes below read them side by side)
+  float term[ORDERED ? 3 : 1][ORDERED ? 43 : 1];
   double acc[NA];
-  uint8_t tag[32];
 };
 
 // Small calls: one warp per atom, every atom of the batch in flight at once.  Lanes
 // are added in FP64 by exchange.  (LJ, 256 atoms, FP64: 10.1 us against 57.4 us with
 // four lanes walking an atom's rows in turn.)
+//
+// Bound by latency (the gathering's loads, then shared memory), so by the warps in
+// flight: only the pairs themselves are kept, as displacements (19 KB a block in FP32,
+// 26 in FP64), and 7 (FP64: 6) blocks per SM are asked for, 72 (80) registers.  A whole
+// call in us with everything kept and 5 blocks, with 7 (6), and with the four lanes per
+// atom before both: FP32 pair arithmetic, 9,000 argon atoms 115, 110, 143; 20,000 161,
+// 147, 156; 45,000 254, 222, 229; 60,000 312, 270, 270; 47,000 Kob-Andersen atoms 242,
+// 201, 198.  FP64: 30,000 argon atoms 186, 175, 200; 47,000 Kob-Andersen atoms 222, 196,
+// 189.  (5 blocks with the pairs alone: 238 and 222 at 45,000 and 47,000 in FP32.)
+// Tried and dropped: a partial sum's terms packed side by side (273 us for 60,000).
 template <int POT, class R, class P, bool VIR>
-__global__ void __launch_bounds__(32 * kWinWarps)
+__global__ void __launch_bounds__(32 * kWinWarps, sizeof(R) == 4 ? 7 : 6)
     k_pair_warp(BinData b, int64_t n, const double *__restrict__ table, int nsp, double cutoff,
                 int flags, P *forces, P *energies, P *stresses, double *e_half,
                 double *vir_half, const uint8_t *__restrict__ sys_active) {
-  using Warp = PairWarpSmem<R, P, VIR>;
+  using Warp = PairWarpSmem<R, VIR>;
   constexpr bool ORDERED = Warp::ORDERED;
   constexpr int NV = VIR ? 16 : 4;
   extern __shared__ __align__(16) char smem[];
@@ -145,34 +166,56 @@ __global__ void __launch_bounds__(32 * kWinWarps)
   PairSum<POT, R, VIR, false> sum;
   sum.clear();
   float fo = 0.0f;  // ORDERED, lanes 0..11: component lane / 4, partial sum lane % 4
-  WinSmem &S = me.win;
-  window_gather(S, G, b.spos, b.bin_start, w, cutoff, [&](int kept) {
+  PairWin<R> &S = me.win;
+  auto inside = [&](const Cand &c) {  // FP64 decision
+    const int sj = min(max(tag_species(c.w), 0), nsp - 1);
+    return c.d2 < prc2[si * nsp + sj] && !(c.q == p && !(S.jx[c.k] | S.jy[c.k] | S.jz[c.k]));
+  };
+  auto put = [&](int at, const Cand &c) {
+    S.x[at] = (R)c.dx;
+    S.y[at] = (R)c.dy;
+    S.z[at] = (R)c.dz;
+    S.info[at] = (uint16_t)(min(max(tag_species(c.w), 0), nsp - 1) | ((c.q - S.q0[c.k]) & 3) << 8);
+  };
+  window_gather(S, G, b.spos, b.bin_start, w, inside, put, [&](int kept) {
     for (int t0 = 0; t0 < kept; t0 += 32) {
       const int t = t0 + lane;
-      float4 term = make_float4(0.f, 0.f, 0.f, 0.f);
+      const bool on = t < kept;
       int share = 0;
-      if (t < kept) {
-        const double dx = S.x[t] - w.x, dy = S.y[t] - w.y, dz = S.z[t] - w.z;
-        const int info = S.info[t], sj = min(info & 255, nsp - 1);
-        share = (info >> 9) & 3;
-        if (dx * dx + dy * dy + dz * dz < prc2[si * nsp + sj] &&  // FP64 decision
-            !(S.q[t] == p && (info & 256))) {
-          const R fr = sum.template add<!ORDERED>(true, (R)dx, (R)dy, (R)dz,
-                                                  prm[si * nsp + sj], prm[sj * nsp + si]);
-          if constexpr (ORDERED) term = make_float4((float)dx, (float)dy, (float)dz, fr);
+      if (on) {
+        const R rx = S.x[t], ry = S.y[t], rz = S.z[t];
+        const int info = S.info[t], sj = info & 255;
+        share = info >> 8;
+        const R fr = sum.template add<!ORDERED>(true, rx, ry, rz, prm[si * nsp + sj],
+                                                prm[sj * nsp + si]);
+        if constexpr (ORDERED) {
+          me.term[0][lane] = __fmul_rn(fr, rx);
+          me.term[1][lane] = __fmul_rn(fr, ry);
+          me.term[2][lane] = __fmul_rn(fr, rz);
         }
       }
       if constexpr (ORDERED) {
-        __syncwarp();
-        me.term[lane] = term;
-        me.tag[lane] = (uint8_t)share;
+        // a partial sum's pairs: a mask of lanes, taken from the lowest up
+        unsigned todo = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned m = __ballot_sync(full, on && share == k);
+          if ((lane & 3) == k) todo = m;
+        }
         __syncwarp();
         if (lane < 12) {
-          const int c = min(kept - t0, 32);
-          const float *d = &me.term[0].x + lane / 4;
-          for (int k = 0; k < c; ++k)
-            if (me.tag[k] == (lane & 3)) fo = __fsub_rn(fo, __fmul_rn(me.term[k].w, d[4 * k]));
+          const float *d = me.term[lane >> 2];
+          while (todo) {
+            const int k0 = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int k1 = todo ? __ffs(todo) - 1 : k0;  // (two reads in flight)
+            const float d0 = d[k0], d1 = d[k1];
+            fo = __fsub_rn(fo, d0);
+            if (todo) fo = __fsub_rn(fo, d1);
+            todo &= todo - 1;
+          }
         }
+        __syncwarp();
       }
     }
   });
@@ -204,8 +247,9 @@ __global__ void __launch_bounds__(32 * kWinWarps)
 // the table stays in registers.
 template <int POT, class R, class P, bool VIR, bool MONO>
 __global__ void __launch_bounds__(32 * kWinWarps, sizeof(R) == 4 ? 6 : 4)
-    k_pair_tile(BinData b, TileList tl, const double *__restrict__ table, int nsp, double cutoff, int flags, P *forces,
-                P *energies, P *stresses, double *e_half, double *vir_half) {
+    k_pair_tile(BinData b, TileList tl, const double *__restrict__ table, int nsp,
+                double cutoff, int flags, P *forces, P *energies, P *stresses, double *e_half,
+                double *vir_half) {
   constexpr bool ROUND = sizeof(R) == 4;  // sums in search order
   extern __shared__ __align__(16) char smem[];
   TileSmem<false> *warps = (TileSmem<false> *)smem;
@@ -258,8 +302,8 @@ __global__ void __launch_bounds__(32 * kWinWarps, sizeof(R) == 4 ? 6 : 4)
           double t[VIR ? 10 : 4] = {(double)sum.fx, (double)sum.fy, (double)sum.fz, sum.ei};
           if constexpr (VIR)
             for (int k = 0; k < 6; ++k) t[4 + k] = sum.v[k];
-          write_atom<P, VIR>(tag_atom(A.w.w), t, flags, b.geom[T.sys].vol, forces, energies, stresses,
-                             e_half, vir_half);
+          write_atom<P, VIR>(tag_atom(A.w.w), t, flags, b.geom[T.sys].vol, forces, energies,
+                             stresses, e_half, vir_half);
         });
   }
 }
@@ -282,41 +326,61 @@ static void carve_pair(Carver &c, PairWork &w, int64_t n, int64_t ns) {
   carve_tiles(c, w.tl, n, ns);
 }
 
-// Up to this many atoms a call takes one warp per atom: fewer tiles than that leave
-// most of the GPU's resident warps idle.  With FP32 pair math the
-// limit is that of the four-lane order of the FP32 sums (k_pair_warp keeps the
-// four-lane order, k_pair_tile the one-lane order that larger calls have).
-constexpr int64_t kPairWarpMaxAtoms = 16384;
+// Up to these many atoms a call takes one warp per atom, beyond them one per tile: a
+// tile is some 190 us of work for its warp whatever the call, so few of them leave the
+// GPU idle.  With FP32 pair math the limit is that of the four-lane order of the sums
+// (k_pair_warp keeps the four-lane order, k_pair_tile the one-lane order that larger
+// calls have).  In FP64, a call in us by warps and by tiles:
+//   one system of argon   18,000 141, 164   30,000 175, 166   45,000 218, 188   60,000 262, 225
+//   the same, soft sphere 18,000 139, 258   30,000 177, 265   45,000 224, 314   60,000 275, 396
+//   copper, 8 to 512 each 18,000  92, 173   29,000 123, 190   46,000 173, 215   62,000 223, 268
+//   Kob-Andersen mixtures 21,000 111, 202   31,000 146, 201   47,000 196, 221   67,000 261, 281
+// The second limit is that of cheap pair functions in systems too large for their tiles
+// to be cut short.
+constexpr int64_t kPairWarpMaxAtoms = kGroupSearchMaxAtoms;
+constexpr int64_t kPairWarpMaxLarge = 24576;
+constexpr int64_t kPairLargeSystem = 4096;
 
 template <int POT, class R, class P, bool VIR>
 static int launch_forces(PairWork &w, int64_t n, int64_t ns, const double *table, int nsp,
                          double cutoff, int flags, P *forces, P *energies, P *stresses,
                          const uint8_t *active, cudaStream_t st) {
-  using Warp = PairWarpSmem<R, P, VIR>;
+  using Warp = PairWarpSmem<R, VIR>;
   const size_t tab = (size_t)nsp * nsp * (sizeof(PairPrm<R>) + sizeof(double));
   auto room = [](auto kernel, size_t bytes) {
     if (bytes > 48 * 1024)
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     return bytes;
   };
-  if (n <= (Warp::ORDERED ? kGroupSearchMaxAtoms : kPairWarpMaxAtoms)) {
+  const bool small_systems = n < kPairLargeSystem * ns;
+  const bool all = Warp::ORDERED || POT == TSB_POT_SOFT || small_systems;
+  if (n <= (all ? kPairWarpMaxAtoms : kPairWarpMaxLarge)) {
     auto kernel = k_pair_warp<POT, R, P, VIR>;
-    kernel<<<grid_for(n, kWinWarps), 32 * kWinWarps, 
+    kernel<<<grid_for(n, kWinWarps), 32 * kWinWarps,
              room(kernel, kWinWarps * sizeof(Warp) + tab), st>>>(
         w.b, n, table, nsp, cutoff, flags, forces, energies, stresses, w.e_half, w.vir_half,
         active);
   } else {
-    TSB_TRY(window_tiles(w.b, n, ns, active, w.tl, st));
     auto go = [&](auto kernel) {
       const size_t bytes = room(kernel, kWinWarps * sizeof(TileSmem<false>) + tab);
-      kernel<<<tile_grid(kernel, bytes), 32 * kWinWarps, bytes, st>>>(
-          w.b, w.tl, table, nsp, cutoff, flags, forces, energies, stresses, w.e_half,
-          w.vir_half);
+      const unsigned grid = tile_grid(kernel, bytes);
+      // Batches of small systems take tiles of 16 atoms while those make at most two
+      // rounds of the resident warps (FP32 113,664 atoms, FP64 75,776): half the work
+      // for a warp where there are warps to spare.  Tiles of 16 and of 32, us: FP32,
+      // copper of 70,000 atoms 259, 285, of 105,000 277, 305, of 131,000 313, 324, of
+      // 197,000 412, 355; Kob-Andersen of 75,000 313, 305, of 85,000 320, 328, of 113,000
+      // 338, 386, of 211,000 522, 432; FP64, Kob-Andersen of 67,000 239, 285, of 85,000
+      // 281, 299, of 113,000 323, 318.  One large system: argon of 70,000 296, 272.
+      const int width = small_systems && n <= (int64_t)32 * kWinWarps * grid ? 16 : 32;
+      TSB_TRY(window_tiles(w.b, n, ns, active, width, w.tl, st));
+      kernel<<<grid, 32 * kWinWarps, bytes, st>>>(w.b, w.tl, table, nsp, cutoff, flags, forces,
+                                                  energies, stresses, w.e_half, w.vir_half);
+      return TSB_OK;
     };
     if (nsp == 1)
-      go(k_pair_tile<POT, R, P, VIR, true>);
+      TSB_TRY(go(k_pair_tile<POT, R, P, VIR, true>));
     else
-      go(k_pair_tile<POT, R, P, VIR, false>);
+      TSB_TRY(go(k_pair_tile<POT, R, P, VIR, false>));
   }
   TSB_CHECK_LAUNCH();
   return TSB_OK;

@@ -310,7 +310,7 @@ static int nl_build(const P *pos, const P *cell, const uint8_t *pbc, const int64
   if (small) {
     k_nl_warp<P, false><<<grid, threads, 0, st>>>(w.b, n, cutoff, flags, w.cnt, out);
   } else {
-    TSB_TRY(window_tiles(w.b, n, ns, nullptr, w.tl, st));
+    TSB_TRY(window_tiles(w.b, n, ns, nullptr, 32, w.tl, st));
     k_nl_wraps<<<grid_for(n), kBlock, 0, st>>>(w.b.sidx, w.b.wrap, n, w.wraps);
     half ? tile_pass(k_nl_tile<P, false, true>) : tile_pass(k_nl_tile<P, false, false>);
   }

@@ -41,14 +41,24 @@ namespace tsb {
 constexpr int kWinWarps = 4;  // warps per block
 
 // ------------------------------------------------------------- one warp per atom
-struct WinSmem {
+// spans of the current run
+struct WinSpans {
+  double sx[32], sy[32], sz[32];
+  int32_t q0[32], pre[32], jx[32], jy[32], jz[32];
+};
+
+struct WinSmem : WinSpans {
   static constexpr int kCap = 192;  // kept candidates (more: several chunks)
   double x[kCap], y[kCap], z[kCap];
   int32_t q[kCap];     // slot (bin order)
-  int32_t info[kCap];  // species | (unshifted) << 8 | (offset in its span & 3) << 9
+  int32_t info[kCap];  // species | (unshifted) << 8
   int32_t ix[kCap], iy[kCap], iz[kCap];  // image
-  double sx[32], sy[32], sz[32];         // spans of the current run
-  int32_t q0[32], pre[32], jx[32], jy[32], jz[32];
+};
+
+// a candidate: shifted position, its distance from the atom, tag, slot and span
+struct Cand {
+  double px, py, pz, dx, dy, dz, d2, w;
+  int q, k;
 };
 
 // window of one position: bins lo..hi per axis, unbounded on periodic axes
@@ -91,15 +101,16 @@ __device__ __forceinline__ Span span_at(const SysGeom &G, const int64_t *__restr
   return s;
 }
 
-// Gather the candidates of the atom at w and call process(n) on the warp for every
-// full chunk and the last one (also when it is empty).  32 spans at a time are
-// laid end to end and lane t of a step takes candidate t of the run, so lanes stay
-// full whatever the spans' lengths.
-template <class F>
-__device__ __forceinline__ void window_gather(WinSmem &S, const SysGeom &G,
+// Gather the candidates of the atom at w that keep(c) takes, put(at, c) each in its
+// place and call process(n) on the warp for every full chunk and the last one (also
+// when it is empty).  32 spans at a time are laid end to end and lane t of a step takes
+// candidate t of the run, so lanes stay full whatever the spans' lengths.
+template <class Smem, class K, class T, class F>
+__device__ __forceinline__ void window_gather(Smem &S, const SysGeom &G,
                                               const double4 *__restrict__ spos,
                                               const int64_t *__restrict__ bin_start,
-                                              const double4 &w, double cutoff, F &&process) {
+                                              const double4 &w, K &&keep_, T &&put,
+                                              F &&process) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned le = 0xffffffffu >> (31 - lane), lt = le >> 1;
@@ -111,7 +122,6 @@ __device__ __forceinline__ void window_gather(WinSmem &S, const SysGeom &G,
   int lo[3], hi[3];
   frame_coords(G, w.x, w.y, w.z, u);
   window_of(G, u, lo, hi);
-  const double reach2 = cutoff * cutoff * (1.0 + 1e-12);
   const int nx = hi[0] - lo[0] + 1, ny = hi[1] - lo[1] + 1;
   const int iz_lo = G.per[2] ? floordiv_dev(lo[2], G.nb[2]) : 0;
   const int nzs = G.per[2] ? floordiv_dev(hi[2], G.nb[2]) - iz_lo + 1 : (hi[2] >= lo[2]);
@@ -121,7 +131,7 @@ __device__ __forceinline__ void window_gather(WinSmem &S, const SysGeom &G,
   int begun = 0;  // spans of the run that start before candidate t0
   bool more = n_spans > 0;
   do {
-    while (more && kept <= WinSmem::kCap - 64) {
+    while (more && kept <= Smem::kCap - 64) {
       if (t0 >= total) {
         base += 32;
         if (base >= n_spans) {
@@ -179,28 +189,22 @@ __device__ __forceinline__ void window_gather(WinSmem &S, const SysGeom &G,
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        double px = 0.0, py = 0.0, pz = 0.0;
+        Cand c{};
         if (in[h]) {
-          px = o[h].x + S.sx[k[h]];
-          py = o[h].y + S.sy[k[h]];
-          pz = o[h].z + S.sz[k[h]];
-          const double dx = px - w.x, dy = py - w.y, dz = pz - w.z;
-          in[h] = dx * dx + dy * dy + dz * dz < reach2;
+          c.px = o[h].x + S.sx[k[h]];
+          c.py = o[h].y + S.sy[k[h]];
+          c.pz = o[h].z + S.sz[k[h]];
+          c.dx = c.px - w.x;
+          c.dy = c.py - w.y;
+          c.dz = c.pz - w.z;
+          c.d2 = c.dx * c.dx + c.dy * c.dy + c.dz * c.dz;
+          c.w = o[h].w;
+          c.q = q[h];
+          c.k = k[h];
+          in[h] = keep_(c);
         }
         const unsigned keep = __ballot_sync(full, in[h]);
-        if (in[h]) {
-          const int at = kept + __popc(keep & lt), kk = k[h];
-          S.x[at] = px;
-          S.y[at] = py;
-          S.z[at] = pz;
-          S.q[at] = q[h];
-          const int ii = S.jx[kk], jj = S.jy[kk], ll = S.jz[kk];
-          S.info[at] = min(max(tag_species(o[h].w), 0), 255) | ((ii | jj | ll) == 0 ? 256 : 0) |
-                       (((q[h] - S.q0[kk]) & 3) << 9);
-          S.ix[at] = ii;
-          S.iy[at] = jj;
-          S.iz[at] = ll;
-        }
+        if (in[h]) put(kept + __popc(keep & lt), c);
         kept += __popc(keep);
       }
       t0 += 64;
@@ -210,6 +214,29 @@ __device__ __forceinline__ void window_gather(WinSmem &S, const SysGeom &G,
     __syncwarp();
     kept = 0;
   } while (more);
+}
+
+// every candidate within the cutoff (and its rounding), with all that is known of it
+template <class F>
+__device__ __forceinline__ void window_gather(WinSmem &S, const SysGeom &G,
+                                              const double4 *__restrict__ spos,
+                                              const int64_t *__restrict__ bin_start,
+                                              const double4 &w, double cutoff, F &&process) {
+  const double reach2 = cutoff * cutoff * (1.0 + 1e-12);
+  window_gather(
+      S, G, spos, bin_start, w, [&](const Cand &c) { return c.d2 < reach2; },
+      [&](int at, const Cand &c) {
+        S.x[at] = c.px;
+        S.y[at] = c.py;
+        S.z[at] = c.pz;
+        S.q[at] = c.q;
+        const int ii = S.jx[c.k], jj = S.jy[c.k], ll = S.jz[c.k];
+        S.info[at] = min(max(tag_species(c.w), 0), 255) | ((ii | jj | ll) == 0 ? 256 : 0);
+        S.ix[at] = ii;
+        S.iy[at] = jj;
+        S.iz[at] = ll;
+      },
+      process);
 }
 
 // ------------------------------------------------------------ a tile per warp
