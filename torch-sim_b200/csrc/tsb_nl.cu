@@ -286,10 +286,22 @@ static void carve_nl(Carver &c, NlWork &w, int64_t n, int64_t ns) {
   w.wraps = c.take<int4>(n);
 }
 
-// Lists of at most this many atoms take one warp per atom: 16384 / 32 tiles would
-// leave most of the GPU's ~3,500 resident warps idle.  (256 atoms: 20 us for both
-// passes, 276 us with one thread per atom.)
-constexpr int64_t kNlWarpMaxAtoms = 16384;
+// Up to these many atoms a list takes one warp per atom, beyond them one per tile: a tile
+// is some 200 us of work for its warp in the two passes whatever the call, so few of them
+// leave the GPU idle.  A whole call in us by warps and by tiles (full lists; half lists
+// change over at the same size or some 15 % later), and by one thread per atom before both:
+//   one system of argon    17,000 264, 335, 505   25,000 319, 351, 554   32,000 361, 331, 571
+//                          45,000 437, 343, 639
+//   copper, 8 to 512 each  17,000 274, 370, 522   32,000 377, 428, 573   45,000 463, 484, 622
+//                          60,000 553, 453, 698
+//   Kob-Andersen density,  18,000 541, 735, 1109  32,000 773, 740, 1371  45,000 997, 1052, 1821
+//   64 to 1,000 each       60,000 1258, 1135, 2018
+// Tiles of a large system are all full and alike; small systems cut theirs short and give
+// windows of many short spans.  (256 atoms: 20 us for both passes, 276 us with one thread
+// per atom.)
+constexpr int64_t kNlWarpMaxAtoms = 49152;
+constexpr int64_t kNlWarpMaxLarge = 28672;
+constexpr int64_t kNlLargeSystem = 4096;  // mean size from which the second limit holds
 
 template <class P>
 static int nl_build(const P *pos, const P *cell, const uint8_t *pbc, const int64_t *sys,
@@ -299,7 +311,7 @@ static int nl_build(const P *pos, const P *cell, const uint8_t *pbc, const int64
   // n bounds the largest system, so a small call takes the one-launch binning
   TSB_TRY(prepare_bins_any<P>(pos, cell, pbc, sys, n, ns, cutoff, w.b, st, nullptr, n));
   const NlOut<P> out{w.off, cap, packed, mapping, stride, sysmap, shifts};
-  const bool small = n <= kNlWarpMaxAtoms;
+  const bool small = n <= (n < kNlLargeSystem * ns ? kNlWarpMaxAtoms : kNlWarpMaxLarge);
   constexpr int threads = 32 * kWinWarps;
   const unsigned grid = grid_for(n, kWinWarps);
   auto tile_pass = [&](auto kernel) {
