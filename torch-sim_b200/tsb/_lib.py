@@ -212,8 +212,11 @@ _MAX_SYS: dict = {}  # id of a tensor -> (weak reference, version, length, syste
 
 def max_system_atoms(system_idx: torch.Tensor, n_systems: int) -> int:
     """Largest system's atom count, kept for a tensor as long as it lives and is not
-    written to (one device read when it changes).  The entry belongs to the tensor
-    itself: an address says nothing once its tensor is gone and another lies there."""
+    written to (one device read when it changes; none for a single system).  The entry
+    belongs to the tensor itself: an address says nothing once its tensor is gone and
+    another lies there."""
+    if n_systems == 1:
+        return system_idx.shape[0]
     key = id(system_idx)
     now = (system_idx._version, system_idx.shape[0], n_systems)
     hit = _MAX_SYS.get(key)
