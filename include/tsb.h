@@ -418,9 +418,10 @@ int tsb_adj_kick(double *lam_p, const double *lam_q, const double *inv_m, double
  * `first`: traj starts at step 0, whose coefficient is dt / 2).  *status (int32, the
  * caller's, zero before) becomes the neighbour count that exceeded max_neighbors, or
  * 1 << 30 for a narrower cell or a system of more than max_system_atoms atoms (such a
- * system's q_out and p_out are its q and p); the results are then meaningless.  max_system_atoms sizes the blocks: it
- * may be larger than the largest system, and a larger system is left out whole.  TSB_ERR_CAPACITY: the
- * lists do not fit a block's shared memory; TSB_ERR_UNSUPPORTED: too many atoms. */
+ * system's q_out and p_out are its q and p); the results are then meaningless.
+ * max_system_atoms sizes the blocks: it may be larger than the largest system, and a
+ * larger system is left out whole.  TSB_ERR_CAPACITY: the lists do not fit a block's
+ * shared memory; TSB_ERR_UNSUPPORTED: too many atoms. */
 int tsb_adj_block_max_atoms(void);
 /* the longest lists (max_neighbors) whose block fits the current device's shared memory,
  * for the sweep or the trajectory alone; 0: too many atoms or species */

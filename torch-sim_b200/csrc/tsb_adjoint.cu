@@ -336,8 +336,8 @@ extern "C" int tsb_rdf_hist_grad(const double *positions, const double *cell_row
   cudaStream_t st = (cudaStream_t)stream;
   TSB_TRY(prepare_bins_any<double>(positions, cell_row, pbc, system_idx, n_atoms, n_systems,
                                    r_max, w.b, st, nullptr, max_system_atoms));
-  k_rdf_grad<<<grid_for(n_atoms, kWinWarps), 32 * kWinWarps, 0, st>>>(w.b, n_atoms, r_max, n_bins, width,
-                                                     dl_dhist, grad_positions);
+  k_rdf_grad<<<grid_for(n_atoms, kWinWarps), 32 * kWinWarps, 0, st>>>(
+      w.b, n_atoms, r_max, n_bins, width, dl_dhist, grad_positions);
   TSB_CHECK_LAUNCH();
   return TSB_OK;
 }

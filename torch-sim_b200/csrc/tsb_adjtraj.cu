@@ -12,7 +12,8 @@
 // so nothing but the launches' ends synchronised them.  One block per system removes
 // the launches; what remains is bound by the gathers of neighbour positions from
 // shared memory (random 8-byte reads) and by FP64 issue.  The same loss and gradients:
-// trajectory 2.3 ms, sweep 4.2 ms, 8.1 ms in all against 45.5 ms.
+// trajectory 2.3 ms, sweep 4.2 ms; with the histogram and its gradient (tsb_adjoint.cu,
+// 0.28 and 0.13 ms) 7.3 ms in all against 45.4 ms.
 //
 // Lists.  Entry: neighbour | image code << 11, image S in {-1,0,1}^3 of the build's
 // wrapped positions, within cutoff + skin; every thread of a block agrees to rebuild
@@ -67,11 +68,13 @@ struct BlkSmem {
 
 __host__ __device__ inline size_t blk_bytes(int max_atoms, int stride, int cap, int nsp, int vecs) {
   return sizeof(double) * ((size_t)3 * max_atoms * (3 + vecs) + 18 + 81 + 5 * nsp * nsp) +
-         sizeof(float) * 84 + sizeof(int32_t) * 4 + sizeof(int32_t) * max_atoms + sizeof(uint16_t) * (size_t)stride * cap +
+         sizeof(float) * 84 + sizeof(int32_t) * (4 + max_atoms) +
+         sizeof(uint16_t) * (size_t)stride * cap +
          (size_t)((max_atoms + 15) / 16 * 16);
 }
 
-__device__ inline BlkSmem blk_carve(char *p, int max_atoms, int stride, int cap, int nsp, int vecs) {
+__device__ inline BlkSmem blk_carve(char *p, int max_atoms, int stride, int cap, int nsp,
+                                    int vecs) {
   BlkSmem s;
   double *d = (double *)p;
   auto take = [&](size_t n) {

@@ -490,7 +490,8 @@ __device__ inline void vl_frame(int64_t p, const P *pos, const P *cell_row,
     w[m] = (double)pos[3 * i + m] -
            (W0 * (double)C[m] + W1 * (double)C[3 + m] + W2 * (double)C[6 + m]);
   // (a row of the table whatever the caller gave)
-  const unsigned long long hi = species ? (unsigned long long)min(max(species[i], 0), nsp - 1) : 0ull;
+  const unsigned long long hi =
+      species ? (unsigned long long)min(max(species[i], 0), nsp - 1) : 0ull;
   wpos[p] = make_double4(w[0], w[1], w[2], __longlong_as_double((long long)(hi << 32)));
   wpos32[p] = make_float4((float)w[0], (float)w[1], (float)w[2], __int_as_float((int)hi));
 }

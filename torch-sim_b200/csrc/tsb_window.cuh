@@ -31,7 +31,6 @@
 // paid per bin, and 2 atoms share it), one block of four warps per 2 x 2 x 2 bins
 // with a ballot per 32 candidates (1245 us), notes walked chunk by chunk in search
 // order (295 us, and see SPREAD below).
-//
 #pragma once
 
 #include "tsb_search.cuh"
@@ -335,9 +334,9 @@ struct TileAtom {
 };
 
 // The atoms of a tile (together when they may share a window, else one by one):
-// begin(A) once per batch with the lanes' atoms,
-// process(A, kept, pre2) for every chunk of kept candidates
-// (pre2: the widened cutoff^2; as far below the cutoff^2 a pair is surely inside), end(A) after the last.
+// begin(A) once per batch with the lanes' atoms, process(A, kept, pre2) for every chunk
+// of kept candidates (pre2: the widened cutoff^2; as far below the cutoff^2 a pair is
+// surely inside), end(A) after the last.
 // wraps: the integer wraps by slot, for SHIFT.
 // SPREAD takes the spans in a scattered order (a fixed one, by the window's shape):
 // in search order a chunk is a slab of the window, near some of the atoms and out of
