@@ -100,6 +100,7 @@ class VerletListModel(ModelInterface):
                 and self._seen_pbc.same(state.pbc)):
             return
         dev = pos.device
+        self._key = None  # (until every buffer is there)
         rcs = self.model.cutoff + self.skin
         counts = torch.bincount(sysi, minlength=ns).double()
         self.max_system_atoms = int(counts.max()) if ns else 0
@@ -108,8 +109,7 @@ class VerletListModel(ModelInterface):
         est = int(4.19 * rcs ** 3 * dens * 1.35) + 16
         if not (est < 4096):
             est = 4096
-        self.cap = max(self.max_neighbors, est)
-        self.list = torch.empty(self.cap * n, dtype=torch.int32, device=dev)
+        self._allot(max(self.max_neighbors, est), n, dev)
         self.counts = torch.empty(n, dtype=torch.int32, device=dev)
         self.flags = torch.zeros(2, dtype=torch.int32, device=dev)
         self.ws = torch.empty(L.load().tsb_vlist_workspace_size(n, ns), dtype=torch.uint8,
@@ -118,6 +118,14 @@ class VerletListModel(ModelInterface):
         self._built = False
         self._key, self._seen = key, tuple(map(L.Seen, of))
         self._seen_pbc = L.SeenPbc(state.pbc)
+
+    def _allot(self, cap, n, dev):
+        """Room for ``cap`` neighbours per atom.  The capacity is what the kernels may
+        write, so it changes after the allocation has succeeded; where it does not, the
+        lists that are there (cut short, perhaps) are no good for a later call."""
+        key, self._key = self._key, None
+        self.list = torch.empty(cap * n, dtype=torch.int32, device=dev)
+        self.cap, self._key = cap, key
 
     def _reset(self, n, ns, dev):
         L.call("tsb_vlist_reset", n, ns, L.ptr(self.ws), self.ws.numel(), L.stream_ptr(dev))
@@ -142,8 +150,7 @@ class VerletListModel(ModelInterface):
         if needed >= (1 << 30):
             raise ValueError("VerletListModel needs every periodic cell width >= cutoff + skin")
         dev = state.positions.device
-        self.cap = int(needed * 1.2) + 8
-        self.list = torch.empty(self.cap * state.n_atoms, dtype=torch.int32, device=dev)
+        self._allot(int(needed * 1.2) + 8, state.n_atoms, dev)
         self._reset(state.n_atoms, state.n_systems, dev)
         self._built = False
         if self.sticky is not None:
@@ -226,8 +233,7 @@ class VerletListModel(ModelInterface):
             self._key = None  # (what has been listed is no good for a later call either)
             raise ValueError("VerletListModel needs every periodic cell width >= "
                              "cutoff + skin")
-        self.cap = int(needed * 1.2) + 8
-        self.list = torch.empty(self.cap * n, dtype=torch.int32, device=dev)
+        self._allot(int(needed * 1.2) + 8, n, dev)
         self._reset(n, ns, dev)
         self._built = False
 
@@ -291,11 +297,11 @@ class VerletListModel(ModelInterface):
         if getattr(self, "_s_key", None) == key:
             return
         dev = state.device
+        self._s_key = None  # (until every buffer is there)
         rcs = self.model.cutoff + self.skin
         vol = float(torch.det(state.cell[0].double()).abs())
         est = int(4.2 * rcs ** 3 * n / vol * 1.35) + 16
-        self.s_cap = max(self.max_neighbors, est)
-        self.s_list = torch.empty(self.s_cap * n, dtype=torch.int32, device=dev)
+        self._s_allot(max(self.max_neighbors, est), n, dev)
         self.s_counts = torch.empty(n, dtype=torch.int32, device=dev)
         self.s_ref = torch.empty((n, 3), dtype=torch.float64, device=dev)
         self.s_wraps = torch.empty((n, 3), dtype=torch.int32, device=dev)
@@ -305,6 +311,10 @@ class VerletListModel(ModelInterface):
                                 device=dev)
         self._s_key = key
         self._s_built = False
+
+    def _s_allot(self, cap, n, dev):
+        self.s_list = torch.empty(cap * n, dtype=torch.int32, device=dev)
+        self.s_cap = cap
 
     def _s_check(self, state, pos, cell64):
         L.call("tsb_verlet_check", L.ptr(pos), L.ptr(self.s_ref), L.ptr(self.s_wraps),
@@ -327,9 +337,7 @@ class VerletListModel(ModelInterface):
             if st >= (1 << 30):
                 raise ValueError("VerletListModel needs every periodic cell width >= "
                                  "cutoff + skin")
-            self.s_cap = int(st * 1.2) + 8
-            self.s_list = torch.empty(self.s_cap * state.n_atoms, dtype=torch.int32,
-                                      device=state.device)
+            self._s_allot(int(st * 1.2) + 8, state.n_atoms, state.device)
         self.n_builds += 1
         self._s_built = True
 
