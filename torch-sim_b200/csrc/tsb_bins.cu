@@ -350,8 +350,9 @@ __global__ void k_bin_sort(const int64_t *bin_start, int64_t nbins_total, int32_
 // system does the geometry, the bin assignment, the counting sort and the
 // gather into bin order, so one launch replaces the batch-wide passes and
 // systems not selected keep their bins untouched.  Bin regions are static
-// (system s owns bins [2 lo_s + s, 2 (lo_s + count_s) + s], room for the
-// 2 count_s + 1 bins and the sentinel its grid may use), so no scan over the
+// (a system whose atoms begin at lo owns bins [3 lo, 3 (lo + count)), room for the
+// 2 count bins its grid may use and the sentinel; they follow the atoms, so systems
+// that do not ascend have regions of their own too), so no scan over the
 // batch is needed.  Order inside a bin is ascending atom index, as k_bin_sort
 // gives: atoms are placed a block-sized chunk at a time, one warp after
 // another, each lane taking its slot after the lower lanes with the same bin.
@@ -376,7 +377,7 @@ __global__ void __launch_bounds__(kBlock)
   __syncthreads();
   const int64_t start = G.start;
   const int nbins = G.nbins;  // <= 2 count
-  const int64_t base = 2 * start + s;
+  const int64_t base = 3 * start;
   const bool small = count <= kSysBinMaxAtoms;
   int32_t *cur = small ? cur_s : b.bin_count + base;
   int32_t *lbin_g = b.bin_of + start;
@@ -467,7 +468,8 @@ int prepare_bins_any(const P *positions, const P *cell_row, const uint8_t *pbc,
                      const int64_t *system_idx, int64_t n, int64_t ns, double cutoff,
                      BinData &b, cudaStream_t st, const int32_t *species,
                      int64_t max_system_atoms) {
-  if (max_system_atoms > 0 && max_system_atoms <= kSysBinMaxAtoms)
+  const bool regions = 3 * n < INT32_MAX;  // bins are counted in 32 bits
+  if (max_system_atoms > 0 && max_system_atoms <= kSysBinMaxAtoms && regions)
     return prepare_bins_sys<P>(positions, cell_row, pbc, system_idx, n, ns, cutoff, b, st,
                                species, nullptr);
   return prepare_bins<P>(positions, cell_row, pbc, system_idx, n, ns, cutoff, b, st, species);
@@ -501,7 +503,8 @@ void carve_bins(Carver &c, BinData &b, int64_t n, int64_t ns) {
   // (what is zeroed together lies together: one memset each, about 2 us)
   b.bin_count = c.take<int32_t>(2 * b.bcap);
   b.bin_fill = b.bin_count ? b.bin_count + b.bcap : nullptr;
-  b.bin_start = c.take<int64_t>(b.bcap + 1);
+  // (the regions of k_bins_sys reach to 3 n, the batch-wide bins to bcap)
+  b.bin_start = c.take<int64_t>((b.bcap > 3 * n ? b.bcap : 3 * n) + 1);
   b.sys_nbins = c.take<int32_t>(ns);
   b.sys_binoff = c.take<int64_t>(ns + 1);
   b.sys_lo = c.take<int64_t>(2 * ns);

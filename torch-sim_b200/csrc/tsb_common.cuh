@@ -105,7 +105,7 @@ struct BinData {
   int32_t *sidx;        // [N] atom index in bin order
   int32_t *sbin;        // [N] bin of each slot of the bin order
   int32_t *bin_count;   // [Bcap]
-  int64_t *bin_start;   // [Bcap+1]
+  int64_t *bin_start;   // [max(Bcap, 3 N)+1]
   int32_t *bin_fill;    // [Bcap]
   int32_t *sys_nbins;   // [S]
   int64_t *sys_binoff;  // [S+1]
@@ -132,8 +132,8 @@ constexpr int kSysBinMaxAtoms = 4096;
 
 // Per-system binning of the systems with only[s] != 0 (all when only is null),
 // one block each, into the same BinData layout (static bin regions: bin_base =
-// 2 sys_lo + s).  Fast for systems of at most kSysBinMaxAtoms atoms; larger ones
-// are binned correctly but slowly.
+// 3 sys_lo, whatever the order of the systems).  Fast for systems of at most
+// kSysBinMaxAtoms atoms; larger ones are binned correctly but slowly.
 template <class P>
 int prepare_bins_sys(const P *positions, const P *cell_row, const uint8_t *pbc,
                      const int64_t *system_idx, int64_t n_atoms, int64_t n_systems,
