@@ -5,10 +5,10 @@ import numpy as np
 import pytest
 import torch
 
+from tsb import _lib as L
 from tsb import models, neighbors
 from tsb.state import SimState
 
-pytestmark = pytest.mark.gpu
 DEV = "cuda"
 N, LENGTH, CUTOFF = 4, 20.0, 3.0  # 2 x 2 x 2 bins for 4 atoms
 
@@ -30,6 +30,7 @@ def _orders(systems):
         yield np.random.default_rng(seed).permutation(systems)
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("systems", [2, 5, 60, 1000])
 @pytest.mark.parametrize("pbc", [True, False])
 def test_neighbour_list(systems, pbc):
@@ -45,6 +46,7 @@ def test_neighbour_list(systems, pbc):
         assert torch.equal(m1, m) and torch.equal(sh1, sh) and torch.equal(s1, idx1[m1[0]])
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("systems", [5, 60, 1000])
 @pytest.mark.parametrize("lists", [False, True])
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
@@ -64,3 +66,36 @@ def test_forces(systems, lists, precision):
     assert bool((out[0][0] != 0).all())
     for o in out[1:]:
         assert all(torch.equal(a, b) for a, b in zip(o, out[0], strict=True))
+
+
+def test_the_lists_size_hint():
+    up = torch.repeat_interleave(torch.arange(3), torch.tensor([5, 5000, 20]))
+    assert L.list_size_hint(up, 3, 5000) == 5000
+    assert L.list_size_hint(2 - up, 3, 5000) == 4096
+    assert L.list_size_hint(2 - up, 3, 900) == 900
+    assert L.list_size_hint(torch.zeros(5000, dtype=torch.int64), 1, 5000) == 5000
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("filler", [0, 70_000])
+def test_lists_of_large_systems(precision, filler):
+    """(the batch-wide bins against those of one block per system: the same bits)"""
+    from test_gpu_vlist_frozen import _batch as batch
+    from test_gpu_vlist_frozen import _into, _model
+
+    sizes = [300, 4500, 900] + [700] * (filler // 700)
+    rest = list(range(3, len(sizes)))
+    starts = [sum(sizes[:k]) for k in range(len(sizes))]
+    st, model = batch(sizes), _model(precision)
+    for order in ([2, 0, 1], [1, 0, 2], [2, 1, 0]):
+        rows = torch.cat([torch.arange(starts[k], starts[k] + sizes[k])
+                          for k in order + rest]).cuda()
+        other, again = batch(sizes, order + rest), _model(precision)
+        st.positions[:] = batch(sizes).positions
+        for _ in range(3):
+            want, got = _into(model, st, None), _into(again, other, None)
+            assert torch.equal(got[0], want[0]) and torch.equal(got[2], want[2])
+            assert torch.equal(got[1], want[1][rows])
+            st.positions[:300] += 0.7  # (one system's lists expire)
+            other.positions[:] = st.positions[rows]

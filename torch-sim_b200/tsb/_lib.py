@@ -232,6 +232,16 @@ def max_system_atoms(system_idx: torch.Tensor, n_systems: int) -> int:
     return value
 
 
+def list_size_hint(system_idx: torch.Tensor, n_systems: int, largest: int) -> int:
+    """``largest`` (the atom count of the largest system) as tsb_vlist_build takes it.  A
+    list's slots lie as the atoms do, the batch-wide bins as the systems are numbered: where
+    the numbers do not ascend, systems are binned one block each whatever their size."""
+    each = 4096  # up to here that is the way anyway
+    if largest > each and n_systems > 1 and bool((system_idx[1:] < system_idx[:-1]).any()):
+        return each
+    return largest
+
+
 class Seen:
     """A tensor that something was worked out for.  The tensor is held, so its memory is
     not handed to another one meanwhile: what has its address and shape is the same data,

@@ -172,6 +172,7 @@ class _ListForces:
         counts = torch.bincount(P.system_idx, minlength=ns).double()
         vol = torch.linalg.det(P.cell_row).abs().clamp_min(1e-30)
         dens = float((counts / vol).max())
+        self.max_sys = L.list_size_hint(P.system_idx, ns, P.max_sys)
         self.cap = max(cap, min(4096, int(4.19 * rcs ** 3 * dens * 1.35) + 16))
         self.list = torch.empty(self.cap * n, dtype=torch.int32, device=dev)
         self.counts = torch.empty(n, dtype=torch.int32, device=dev)
@@ -192,7 +193,7 @@ class _ListForces:
                self.ws.numel(), st)
         L.call("tsb_vlist_build", L.ptr(q), L.ptr(P.cell_row), L.ptr(P.pbc),
                L.ptr(P.system_idx), L.ptr(P.species), n, ns, L.F64, P.cutoff, self.skin,
-               L.ptr(self.list), L.ptr(self.counts), self.cap, P.max_sys, L.ptr(self.flags),
+               L.ptr(self.list), L.ptr(self.counts), self.cap, self.max_sys, L.ptr(self.flags),
                L.ptr(self.ws), self.ws.numel(), st)
         torch.maximum(self.sticky, self.flags[1:], out=self.sticky)
 

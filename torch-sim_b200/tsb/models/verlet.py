@@ -103,7 +103,7 @@ class VerletListModel(ModelInterface):
         self._key = None  # (until every buffer is there)
         rcs = self.model.cutoff + self.skin
         counts = torch.bincount(sysi, minlength=ns).double()
-        self.max_system_atoms = int(counts.max()) if ns else 0
+        self.max_system_atoms = L.list_size_hint(sysi, ns, int(counts.max()) if ns else 0)
         vol = torch.linalg.det(cell_row.double()).abs().clamp_min(1e-30)
         dens = float((counts / vol).max())
         est = int(4.19 * rcs ** 3 * dens * 1.35) + 16
