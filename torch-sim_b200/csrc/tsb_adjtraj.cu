@@ -56,7 +56,7 @@ struct BlkSmem {
   double *wx, *wy, *wz;  // W C of each atom's wrap at the build
   double *vx, *vy, *vz;  // sweep: lam_p, the vector the Hessian acts on
   double *lx, *ly, *lz;  // sweep: lam_q
-  double *C, *T;         // row cell; fractional u_k = T[k] . x (columns of T) [9] each
+  double *C, *T;         // row cell, its inverse (u_k = sum_m x_m T[3 m + k]) [9] each
   double *sv;            // [27][3] S C
   float *svf;            // the same in FP32
   int32_t *per;          // [3] periodic axes, [1] the lists can hold the cell's pairs
@@ -142,14 +142,15 @@ struct BlkThread {
                        C[2] * (C[3] * C[7] - C[4] * C[6]);
       const bool frac = isfinite(d) && fabs(d) > 1e-12;
       const double id = frac ? 1.0 / d : 0.0;
+      // the inverse of the row cell, row-major
       T[0] = (C[4] * C[8] - C[5] * C[7]) * id;
-      T[3] = (C[2] * C[7] - C[1] * C[8]) * id;
-      T[6] = (C[1] * C[5] - C[2] * C[4]) * id;
-      T[1] = (C[5] * C[6] - C[3] * C[8]) * id;
+      T[1] = (C[2] * C[7] - C[1] * C[8]) * id;
+      T[2] = (C[1] * C[5] - C[2] * C[4]) * id;
+      T[3] = (C[5] * C[6] - C[3] * C[8]) * id;
       T[4] = (C[0] * C[8] - C[2] * C[6]) * id;
-      T[7] = (C[2] * C[3] - C[0] * C[5]) * id;
-      T[2] = (C[3] * C[7] - C[4] * C[6]) * id;
-      T[5] = (C[1] * C[6] - C[0] * C[7]) * id;
+      T[5] = (C[2] * C[3] - C[0] * C[5]) * id;
+      T[6] = (C[3] * C[7] - C[4] * C[6]) * id;
+      T[7] = (C[1] * C[6] - C[0] * C[7]) * id;
       T[8] = (C[0] * C[4] - C[1] * C[3]) * id;
       int fits = 1;
       for (int k = 0; k < 3; ++k) {
